@@ -54,6 +54,7 @@ extern "C" emp_status emp_puzzle_create(const emp_puzzle_desc* desc, emp_puzzle*
     else p->order = emp::order_basic(desc->width, desc->height);
     if (!emp::build_plan(p->model, p->order, p->plan, err)) return fail(EMP_ERR_INVALID, "emp_puzzle_create: " + err);
     emp::build_device_tables(p->model, p->plan, p->tables);
+    p->compact = emp::build_compact(p->model, p->plan);
     for (uint32_t k = 0; k < 3; ++k)
         for (uint32_t e = 0; e < 4 * p->model.nb_kind(k); ++e)
             p->extra_count += (p->tables.blob[p->tables.tinfo_off[k] + e] >> 20) & 1u;
@@ -355,6 +356,31 @@ emp_status resume_records(const emp_puzzle_t& pz, const uint16_t* situation, uin
     return EMP_OK;
 }
 
+// Decides for the compact search and uploads its tables: every puzzle of the plan has them,
+// and in a plan of several puzzles every centre space is one word.  Measured on a B200, batches
+// of sides 4..9 in 2 s: with one 9x9 puzzle of two words the whole plan runs the two-word kernel
+// from tables in global memory, 1.7e10 to 2.4e10 placements/s against 2.7e10 of the bitfield
+// search; sides up to 8, one word each, 6.8e10 against 3.1e10.
+emp_status upload_compact(emp_bt_plan_t& pl)
+{
+    pl.compact = pl.cfg.stack_placement == 0;
+    for (emp_puzzle p : pl.puzzles)
+        if (p->compact.empty() || (pl.puzzles.size() > 1 && p->compact[0] != 1)) pl.compact = false;
+    if (!pl.compact) return EMP_OK;
+    std::vector<uint32_t> blob;
+    std::vector<uint64_t> offs;
+    for (emp_puzzle p : pl.puzzles) {
+        offs.push_back(blob.size());  // multiples of 4 words: 16-byte aligned
+        blob.insert(blob.end(), p->compact.begin(), p->compact.end());
+    }
+    std::memcpy(&pl.chdr, blob.data(), sizeof(pl.chdr));
+    CUDA_TRY(pl.ctables.alloc(sizeof(uint32_t) * blob.size()));
+    CUDA_TRY(pl.coff.alloc(sizeof(uint64_t) * offs.size()));
+    CUDA_TRY(cudaMemcpy(pl.ctables.p, blob.data(), sizeof(uint32_t) * blob.size(), cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMemcpy(pl.coff.p, offs.data(), sizeof(uint64_t) * offs.size(), cudaMemcpyHostToDevice));
+    return EMP_OK;
+}
+
 emp_status create_plan(const emp_puzzle* puzzles, uint32_t count, const emp_bt_config* config, bool dump,
                        emp_bt_plan* out, const ResumeSpec* resume)
 {
@@ -423,8 +449,14 @@ emp_status create_plan(const emp_puzzle* puzzles, uint32_t count, const emp_bt_c
     } else {
         EMP_TRY(expand(*pl));
     }
+    // The compact search takes plans whose stack placement is left to the library and whose
+    // puzzles all have compact tables (row-major orders whose pieces fit its slots); an explicit
+    // placement and the other orders run dfs_kernel / dfs_warp_kernel.
+    if (pl->cfg.stack_placement > 4)
+        return fail(EMP_ERR_INVALID, "stack_placement must be 0 (default), 1, 2, 3 or 4");
+    EMP_TRY(upload_compact(*pl));
     // hot tables in shared memory when the plan holds one puzzle
-    const uint32_t hot = (pl->puzzles[0]->tables.blob[26] + 3u) & ~3u;
+    const uint32_t hot = pl->compact ? pl->chdr.hot : (pl->puzzles[0]->tables.blob[26] + 3u) & ~3u;
     const bool want_smem = pl->cfg.table_placement == 2 || (pl->cfg.table_placement == 0 && count == 1);
     pl->smem_tab_words = (want_smem && count == 1 && hot * 4 <= 64 * 1024) ? hot : 0;
     if (pl->cfg.table_placement == 2 && !pl->smem_tab_words)
@@ -432,15 +464,12 @@ emp_status create_plan(const emp_puzzle* puzzles, uint32_t count, const emp_bt_c
     // launch geometry: the block size with the most resident warps per SM
     cudaDeviceProp prop;
     CUDA_TRY(cudaGetDeviceProperties(&prop, pl->device));
-    if (pl->cfg.stack_placement > 4)
-        return fail(EMP_ERR_INVALID, "stack_placement must be 0 (default), 1, 2, 3 or 4");
-    // default: the shared 32-bit stack next to staged tables (a single puzzle) while it
-    // leaves at least 16 warps per SM, else the global stack.  Measured on a B200: 8x8
-    // 2.7e10 placements/s shared against 2.0e10 global; 12x12 (8 warps per SM shared)
-    // 1.8e10 against 2.3e10; the 4096-instance batch (tables in global memory) 2.2e10
-    // against 2.7e10.
+    // default of the bitfield search: the shared 32-bit stack next to staged tables (a single
+    // puzzle) while it leaves at least 16 warps per SM, else the global stack.  Measured on a
+    // B200: 12x12 (8 warps per SM shared) 1.8e10 against 2.3e10.  The compact search (one word a
+    // level) starts from the shared stack for batches too, and keeps it down to 8 warps there.
     const bool default_stack = pl->cfg.stack_placement == 0;
-    pl->stack_mode = default_stack ? (pl->smem_tab_words ? emp::kStackShared32 : emp::kStackGlobal32)
+    pl->stack_mode = default_stack ? (pl->smem_tab_words || pl->compact ? emp::kStackShared32 : emp::kStackGlobal32)
                                    : static_cast<int>(pl->cfg.stack_placement);
     std::vector<uint32_t> candidates;
     if (pl->cfg.threads_per_block) candidates.push_back(pl->cfg.threads_per_block);
@@ -450,14 +479,29 @@ emp_status create_plan(const emp_puzzle* puzzles, uint32_t count, const emp_bt_c
     auto pick_geometry = [&]() -> emp_status {
         best_warps = 0;
         for (uint32_t threads : candidates) {
-            const void* fn = emp::dfs_kernel_symbol(pl->max_kw, pl->smem_tab_words != 0, threads, pl->stack_mode);
+            const bool gs = pl->stack_mode == emp::kStackGlobal32;
+            const void* fn =
+                pl->compact ? emp::compact_kernel_symbol(pl->chdr.nw, pl->smem_tab_words != 0, gs, threads)
+                            : emp::dfs_kernel_symbol(pl->max_kw, pl->smem_tab_words != 0, threads, pl->stack_mode);
             if (!fn) return fail(EMP_ERR_INVALID, "threads_per_block must be 128, 256 or 512");
             const size_t smem =
-                emp::dfs_smem_bytes(pl->max_levels, pl->max_avail, threads, pl->smem_tab_words, pl->stack_mode);
+                pl->compact
+                    ? emp::compact_smem_bytes(pl->max_levels, threads, pl->smem_tab_words, gs)
+                    : emp::dfs_smem_bytes(pl->max_levels, pl->max_avail, threads, pl->smem_tab_words, pl->stack_mode);
             if (smem > static_cast<size_t>(prop.sharedMemPerBlockOptin)) continue;
-            CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+            // (the compact kernel's limit and carve-out are the same for every plan, so that a plan
+            // created later never lowers them under an earlier one)
+            CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          static_cast<int>(pl->compact ? prop.sharedMemPerBlockOptin : smem)));
+            if (pl->compact && !gs && !pl->smem_tab_words)
+                CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 44));
             int per_sm = 0;
             CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, static_cast<int>(threads), smem));
+            // compact tables in global memory want L1 for themselves: stacks get 100 KB of the 228
+            // (44 %).  Measured on a B200, 665 8x8 instances: 1.06e11 placements/s with 100 KB of
+            // stacks (12 warps), 8.0e10 with 132 KB, 6.5e10 with 164 KB, 7.4e10 with 28 warps' 210 KB
+            if (pl->compact && !gs && !pl->smem_tab_words)
+                per_sm = std::min<int>(per_sm, std::max<int>(1, static_cast<int>(100 * 1024 / (smem + 1024))));
             if (pl->cfg.blocks_per_sm) per_sm = std::min<int>(per_sm, static_cast<int>(pl->cfg.blocks_per_sm));
             const int warps = per_sm * static_cast<int>(threads / 32);
             if (per_sm >= 1 && warps > best_warps) {
@@ -469,22 +513,35 @@ emp_status create_plan(const emp_puzzle* puzzles, uint32_t count, const emp_bt_c
         return EMP_OK;
     };
     EMP_TRY(pick_geometry());
-    if (default_stack && pl->stack_mode == emp::kStackShared32 && best_warps < 16) {
+    if (default_stack && pl->stack_mode == emp::kStackShared32 && best_warps < (pl->compact && count > 1 ? 8 : 16)) {
         pl->stack_mode = emp::kStackGlobal32;
         EMP_TRY(pick_geometry());
     }
     if (!best_warps)
         return fail(EMP_ERR_UNSUPPORTED, "per-thread DFS state does not fit shared memory; use fewer threads per block");
-    CUDA_TRY(pl->spill.alloc(sizeof(uint64_t) * static_cast<size_t>(pl->blocks) * pl->threads * pl->max_levels *
-                             pl->max_kw));
-    if (pl->stack_mode == emp::kStackGlobal32)
-        CUDA_TRY(pl->stack.alloc(sizeof(uint32_t) * static_cast<size_t>(pl->blocks) * pl->threads * pl->max_levels));
-    // round queues: room for every resident thread to hand back a full path twice
     const uint64_t resident = static_cast<uint64_t>(pl->blocks) * pl->threads;
-    pl->capacity = std::max<uint64_t>(resident * 2 * (pl->max_levels - pl->depth + 1) / 4, 1u << 16);
-    pl->capacity = std::min<uint64_t>(pl->capacity, (uint64_t)1 << 23);
-    CUDA_TRY(pl->rec_a.alloc(sizeof(uint32_t) * pl->rec_words * pl->capacity));
-    CUDA_TRY(pl->rec_b.alloc(sizeof(uint32_t) * pl->rec_words * pl->capacity));
+    if (pl->compact) {
+        if (pl->stack_mode == emp::kStackGlobal32)
+            CUDA_TRY(pl->stack.alloc(sizeof(uint32_t) * resident * emp::compact_stack_levels(pl->max_levels)));
+        // round queues: a thread hands its state back at most once a round, with an item per
+        // level that holds candidates: about 6 on an 8x8 board.  Room for 24; a thread that
+        // finds the queue full keeps its work.
+        pl->queue_words = emp::compact_state_words(pl->max_levels, pl->chdr.nw);
+        pl->capacity = resident * std::min<uint32_t>(24, pl->max_levels);
+        const uint64_t bytes = sizeof(uint32_t) * pl->queue_words * resident + sizeof(uint64_t) * pl->capacity;
+        CUDA_TRY(pl->rec_a.alloc(bytes));
+        CUDA_TRY(pl->rec_b.alloc(bytes));
+    } else {
+        CUDA_TRY(pl->spill.alloc(sizeof(uint64_t) * static_cast<size_t>(resident) * pl->max_levels * pl->max_kw));
+        if (pl->stack_mode == emp::kStackGlobal32)
+            CUDA_TRY(pl->stack.alloc(sizeof(uint32_t) * static_cast<size_t>(resident) * pl->max_levels));
+        // round queues: room for every resident thread to hand back a full path twice
+        pl->queue_words = pl->rec_words;
+        pl->capacity = std::max<uint64_t>(resident * 2 * (pl->max_levels - pl->depth + 1) / 4, 1u << 16);
+        pl->capacity = std::min<uint64_t>(pl->capacity, (uint64_t)1 << 23);
+        CUDA_TRY(pl->rec_a.alloc(sizeof(uint32_t) * pl->queue_words * pl->capacity));
+        CUDA_TRY(pl->rec_b.alloc(sizeof(uint32_t) * pl->queue_words * pl->capacity));
+    }
     // default split budget.  Without a deadline the whole tree gets searched and a small
     // budget shares each round's tail out sooner: measured on a B200 over slices of four
     // 8x8 workload puzzles, 2.68e10 placements/s at 2048 steps, 3.65e10 at 256, 3.79e10
@@ -542,7 +599,7 @@ constexpr uint32_t kMaxRounds = 100000;
 
 // The whole run as one graph:
 //   reset -> zero the queue counters -> DFS round 1 (initial records) -> advance
-//   -> while (records were handed back) { copy them to the input queue -> DFS -> advance }
+//   -> while (records were handed back) { take them as the input -> DFS -> advance }
 // The advance kernel sets the loop's condition on the device, so the host
 // launches the graph once and never waits between rounds.
 emp_status build_graph(emp_bt_plan_t& pl)
@@ -564,7 +621,7 @@ emp_status build_graph(emp_bt_plan_t& pl)
     if (e == cudaSuccess) e = cudaMemsetAsync(pl.counters.p, 0, pl.counters.bytes, cs);
     if (e == cudaSuccess && pl.item_nodes.p) e = cudaMemsetAsync(pl.item_nodes.p, 0, pl.item_nodes.bytes, cs);
     if (e == cudaSuccess && pl.item_sols.p) e = cudaMemsetAsync(pl.item_sols.p, 0, pl.item_sols.bytes, cs);
-    if (e == cudaSuccess) e = emp::launch_dfs(P, pl.blocks, pl.threads, cs);
+    if (e == cudaSuccess) e = pl.launch_round(P, cs);
     if (e == cudaSuccess) e = emp::launch_round_advance(P, loop, kMaxRounds, cs);
     cudaError_t e2 = cudaStreamEndCapture(cs, &g);
     CUDA_TRY(e);
@@ -590,10 +647,17 @@ emp_status build_graph(emp_bt_plan_t& pl)
     CUDA_TRY(cudaGraphAddNode(&cnode, g, &sink, 1, &cp));
     cudaGraph_t body = cp.conditional.phGraph_out[0];
     emp::BtLaunch Q = P;
-    Q.in_rec = pl.rec_a.as<uint32_t>();
+    // the bitfield search reads a copy of the handed-back records; the compact one lets the
+    // two queues change roles
+    if (pl.compact) {
+        Q.swap_rec = pl.rec_a.as<uint32_t>();
+        Q.in_items = 1;
+    } else {
+        Q.in_rec = pl.rec_a.as<uint32_t>();
+    }
     CUDA_TRY(cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    e = emp::launch_round_copy(Q, pl.rec_a.as<uint32_t>(), pl.rec_b.as<uint32_t>(), cs);
-    if (e == cudaSuccess) e = emp::launch_dfs(Q, pl.blocks, pl.threads, cs);
+    e = pl.compact ? cudaSuccess : emp::launch_round_copy(Q, pl.rec_a.as<uint32_t>(), pl.rec_b.as<uint32_t>(), cs);
+    if (e == cudaSuccess) e = pl.launch_round(Q, cs);
     if (e == cudaSuccess) e = emp::launch_round_advance(Q, loop, kMaxRounds, cs);
     e2 = cudaStreamEndCapture(cs, &body);
     CUDA_TRY(e);
@@ -650,7 +714,8 @@ extern "C" emp_status emp_bt_plan_run(emp_bt_plan plan, void* stream)
         P.n_in = n_in;
         P.out_rec = out->as<uint32_t>();
         CUDA_TRY(cudaEventRecord(plan->evr0, st));
-        CUDA_TRY(emp::launch_dfs(P, plan->blocks, plan->threads, st));
+        P.in_items = plan->rounds != 0;
+        CUDA_TRY(plan->launch_round(P, st));
         CUDA_TRY(cudaEventRecord(plan->evr1, st));
         ++plan->rounds;
         unsigned long long tail = 0;

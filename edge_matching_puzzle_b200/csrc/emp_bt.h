@@ -1,6 +1,7 @@
 // Launch interface of the exhaustive backtracker kernels (emp_bt.cu).
 #pragma once
 
+#include "emp_compact.h"
 #include "emp_layout.h"
 
 #include <cuda_runtime.h>
@@ -87,6 +88,17 @@ struct BtLaunch {
     uint32_t first_lock_init = 0;             // value the records' locks start at (1: held by nobody; tests)
     int stack_mode = kStackShared32;          // placement of the per-thread DFS stack (StackMode)
     uint32_t* stack = nullptr;                // kStackGlobal32: [blocks][max_levels][threads] stack entries
+    // the compact search (emp_btc.cu)
+    const uint32_t* ctables = nullptr;        // all compact blobs
+    const uint64_t* coffset = nullptr;        // word offset of each puzzle's blob
+    CompactHeader chdr{};                     // puzzle 0's header (all blobs share nw)
+    int in_items = 0;                         // 1: in_rec holds states and items of the round before,
+                                              // 0: initial records
+    uint32_t crec_words = 0;                  // words per handed-back state
+    uint64_t items_off = 0;                   // word offset of the items behind the states of a queue
+    uint32_t stack_levels = 0;                // levels of a thread's stack column in `stack`
+    uint32_t* swap_rec = nullptr;             // graph runs after the first round: the queue that changes
+                                              // roles with out_rec every round
 };
 
 cudaError_t launch_expand(const BtLaunch& P, const uint16_t* parents, const uint32_t* parent_puzzle,
@@ -129,6 +141,12 @@ cudaError_t launch_solution_index(const SolutionRecord* sols, uint64_t nsol, con
                                   unsigned long long* out, cudaStream_t stream);
 cudaError_t launch_record_prefix(const uint32_t* rec, uint32_t rec_words, uint64_t i, uint16_t* out,
                                  cudaStream_t stream);
+// The compact search: kernels for nw 64-bit words of centre slots (1, 2 or 4).
+const void* compact_kernel_symbol(uint32_t nw, bool smem_tables, bool global_stack, uint32_t threads);
+uint32_t compact_state_words(uint32_t max_levels, uint32_t nw);
+uint32_t compact_stack_levels(uint32_t max_levels);
+size_t compact_smem_bytes(uint32_t max_levels, uint32_t threads, uint32_t tab_words, bool global_stack);
+cudaError_t launch_dfs_compact(const BtLaunch& P, uint32_t blocks, uint32_t threads, cudaStream_t stream);
 const void* dfs_kernel_symbol(uint32_t max_kw, bool smem_tables, uint32_t threads, int stack_mode);
 
 }  // namespace emp

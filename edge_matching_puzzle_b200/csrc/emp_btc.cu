@@ -1,0 +1,782 @@
+// Exhaustive backtracker over the compact search tables (emp_compact.h): the default search
+// of row-major orders.
+//
+// The search and its initial records are those of dfs_kernel (emp_bt.cu); what differs is what a
+// placement costs.  A level's candidates are one row of the tables and the availability, one
+// AND of 64 bits for boards of up to about 62 centre pieces, where dfs_kernel combines three
+// 64-bit words of piece x orientation bits, searches them and keeps a set apart for identical
+// pieces.  Availability stays in registers, and a step looks one level ahead: it takes the
+// next candidate of the level, counts it, and goes down only when that leaves the next level
+// a candidate, so a dead end costs no stack traffic and no step back.
+//
+// A step of a warp runs (1) a pop for the lanes whose level is exhausted, (2) the next candidate
+// for all lanes that have one, (3) the way down for those whose candidate allows it.  A lane
+// whose pop found nothing left there pops again at the next step.  What is rare (flagged rows,
+// solutions) is left to a vote of the warp, so the common path has two divergent regions.  The set left at a level is not stored: a pop recomputes it as
+// the row AND the availability (which is the level's entry availability again) above the
+// slot placed there, with the trials of flagged rows replayed (emp_compact.h).
+//
+// The stack keeps one 32-bit word a level:
+//   south colour | slot << 8 | more << 16 | space << 17 | (byte offset of the row / 16) << 18
+// (more: candidates remained after this one was taken).  A is the availability of the space
+// of the current level and O the other one; they change places when the level's space does.
+//
+// What bounds it: instruction issue (74 % of the slots in the main rounds on a B200, 24 warps
+// an SM, shared-memory latency behind them); 30 of 32 lanes have work at a step, 22 of them a
+// candidate.  Measured, 1/64 of the 8x8 tree of 4 border / 8 interior colours, seed 0
+// (2.77e9 placements): 62.9 ms with dfs_kernel (4.4e10 placements/s), 26.3 ms here (1.05e11/s).
+#include "emp_bt.h"
+
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+namespace emp {
+
+namespace {
+
+constexpr unsigned kFull = 0xFFFFFFFFu;
+
+// Work handed from one round to the next: a thread writes its whole state once, and one item
+// per level of it that still holds candidates.  A state, 32-bit words: [0,1] subtree, [2] level
+// L, [3] puzzle, [4] row of L, [5] first slot left at L, [6,7] border availability, then the
+// centre availability (nw 64-bit words) and the stack words of levels 0..L-1.  An item, 64
+// bits: state << 32 | level (kNoItem: none).
+constexpr unsigned long long kNoItem = ~0ull;
+constexpr uint32_t kEmptyRec = 1u << 17;  // initial records: nothing to search
+__host__ __device__ constexpr uint32_t state_header(uint32_t nw) { return (8 + 2 * nw + 3) & ~3u; }
+
+__device__ __forceinline__ uint64_t global_ns()
+{
+    uint64_t t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+
+extern __shared__ __align__(16) uint32_t g_smem[];
+
+__device__ __forceinline__ uint64_t ldg64(const uint32_t* p)
+{
+    return __ldg(reinterpret_cast<const unsigned long long*>(p));
+}
+
+// bits of `v` at and above bit `s` (0..64)
+__device__ __forceinline__ uint64_t from_bit(uint64_t v, uint32_t s)
+{
+    uint64_t ones;
+    asm("shl.b64 %0, %1, %2;" : "=l"(ones) : "l"(~0ull), "r"(s));  // a shift by 64 gives 0
+    return v & ones;
+}
+
+template <int NW>
+struct Search {
+    uint64_t orig, nodes, sols, steps;
+    const uint32_t* tb;              // the puzzle's blob
+    uint32_t pz, n, L, base, space;
+    int row;                         // byte offset of level L's row
+    int entries;                     // byte offset of its slot 0 entry
+    uint64_t R[NW];                  // candidates left at level L
+    uint64_t A[NW], O[NW];           // availability of level L's space, of the other space
+    bool active;
+};
+
+template <int NW>
+struct Row {
+    uint64_t m[NW];
+    int entries;
+    uint32_t clears;
+};
+
+struct SlotBits {
+    uint64_t toggle, above;
+};
+
+// Table access by byte offset from the blob's start: SM = the plan's single puzzle, hot tables
+// staged in shared memory; otherwise read through the read-only path.
+template <bool SM, int NW>
+struct Tab {
+    using S = Search<NW>;
+    static __device__ __forceinline__ uint4 quad(const S& s, int off)
+    {
+        return SM ? *reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(g_smem) + off)
+                  : __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(s.tb) + off));
+    }
+    static __device__ __forceinline__ uint4 desc(const S& s, uint32_t l) { return quad(s, 4 * kCompactHeader + 16 * l); }
+    static __device__ __forceinline__ SlotBits slot(const BtLaunch& P, const S& s, uint32_t space, uint32_t slot)
+    {
+        const uint32_t at = SM ? 4 * P.chdr.slots : 4 * kCompactHeader + 16 * (s.n + 1);
+        const uint4 v = quad(s, at + 16 * (space * (64 * NW) + slot));
+        return {v.x | static_cast<uint64_t>(v.y) << 32, v.z | static_cast<uint64_t>(v.w) << 32};
+    }
+    static __device__ __forceinline__ Row<NW> row(const S& s, int off)
+    {
+        Row<NW> r;
+        const uint4 v = quad(s, off);
+        r.m[0] = v.x | static_cast<uint64_t>(v.y) << 32;
+        if (NW == 1) {
+            r.entries = v.z;
+            r.clears = v.w;
+        } else {
+            r.m[NW > 1] = v.z | static_cast<uint64_t>(v.w) << 32;
+            uint4 u = quad(s, off + 16);
+            if (NW > 2) {
+                r.m[NW > 2 ? 2 : 0] = u.x | static_cast<uint64_t>(u.y) << 32;
+                r.m[NW > 2 ? 3 : 0] = u.z | static_cast<uint64_t>(u.w) << 32;
+                u = quad(s, off + 32);
+            }
+            r.entries = u.x;
+            r.clears = u.y;
+        }
+        return r;
+    }
+    static __device__ __forceinline__ uint32_t entry(const S& s, int entries, uint32_t slot)
+    {
+        const int off = entries + 2 * static_cast<int>(slot);
+        return SM ? *reinterpret_cast<const uint16_t*>(reinterpret_cast<const char*>(g_smem) + off)
+                  : __ldg(reinterpret_cast<const uint16_t*>(reinterpret_cast<const char*>(s.tb) + off));
+    }
+};
+
+__device__ __forceinline__ uint32_t word_slot(uint32_t w) { return (w >> 8) & 0xFFu; }
+__device__ __forceinline__ bool word_more(uint32_t w) { return (w >> 16) & 1u; }
+__device__ __forceinline__ uint32_t word_space(uint32_t w) { return (w >> 17) & 1u; }
+__device__ __forceinline__ int word_row(uint32_t w) { return static_cast<int>((w >> 14) & 0x3FFF0u); }
+__device__ __forceinline__ uint32_t make_word(uint32_t e, uint32_t slot, bool more, uint32_t space, int row)
+{
+    return ((e >> 9) & 31u) | (slot << 8) | (static_cast<uint32_t>(more) << 16) | (space << 17) |
+           (static_cast<uint32_t>(row) << 14);
+}
+// byte offset of the row at a level with descriptor d: west entry and north colour
+template <int NW>
+__device__ __forceinline__ int row_at(uint4 d, uint32_t west, uint32_t north)
+{
+    return static_cast<int>(d.x) + static_cast<int>((west & d.z & 0x1F0u) * (row_bytes(NW) / 16)) +
+           static_cast<int>(north * d.y);
+}
+__device__ __forceinline__ uint32_t desc_space(uint4 d) { return (d.z >> 16) & 1u; }
+
+template <int NW>
+__device__ __forceinline__ bool any(const uint64_t* r)
+{
+    uint64_t x = r[0];
+#pragma unroll
+    for (int w = 1; w < NW; ++w) x |= r[w];
+    return x != 0;
+}
+
+// lowest slot of a set that is not empty
+template <int NW>
+__device__ __forceinline__ uint32_t first_slot(const uint64_t* r)
+{
+    uint64_t x = r[NW - 1];
+    uint32_t at = 64 * (NW - 1);
+#pragma unroll
+    for (int w = NW - 2; w >= 0; --w)
+        if (r[w]) {
+            x = r[w];
+            at = 64 * w;
+        }
+    return at + static_cast<uint32_t>(__ffsll(static_cast<long long>(x))) - 1;
+}
+
+// A and O for a level of space `space`
+template <int NW>
+__device__ __forceinline__ void to_space(Search<NW>& s, uint32_t space)
+{
+    const bool swap = s.space != space;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+        const uint64_t a = s.A[w], o = s.O[w];
+        s.A[w] = swap ? o : a;
+        s.O[w] = swap ? a : o;
+    }
+    s.space = space;
+}
+
+// the piece of a slot of the current space: placed or given back
+template <int NW>
+__device__ __forceinline__ void toggle(uint64_t* a, uint32_t slot, uint64_t bits)
+{
+#pragma unroll
+    for (int w = 0; w < NW; ++w) a[w] ^= NW == 1 || w == static_cast<int>(slot >> 6) ? bits : 0ull;
+}
+
+// The candidates of a flagged row that the reference tries: in ascending order, each trial
+// taking out what its identical mask removes (emp_position_strategy.h:197-200).
+template <int NW>
+struct Set {
+    uint64_t w[NW];
+};
+
+template <int NW>
+__device__ __forceinline__ Set<NW> replay_trials(const uint32_t* id, Set<NW> left)
+{
+    Set<NW> r{};
+    while (any<NW>(left.w)) {
+        const uint32_t slot = first_slot<NW>(left.w);
+#pragma unroll
+        for (int w = 0; w < NW; ++w) {
+            const uint64_t bit = w == static_cast<int>(slot >> 6) ? 1ull << (slot & 63u) : 0ull;
+            r.w[w] |= bit;
+            left.w[w] &= ~(bit | ldg64(id + 2 * (slot * NW + w)));
+        }
+    }
+    return r;
+}
+
+// leaves the candidates that are tried in `r`, the candidates of a flagged row
+template <int NW>
+__device__ __forceinline__ void only_tried(const uint32_t* id, uint64_t* r)
+{
+    if (NW == 1 && !(r[0] & (r[0] - 1))) return;
+    Set<NW> v;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) v.w[w] = r[w];
+    v = replay_trials<NW>(id, v);
+#pragma unroll
+    for (int w = 0; w < NW; ++w) r[w] = v.w[w];
+}
+
+// the current level's candidates: its row AND the availability, without those that other trials
+// of a flagged row remove
+template <bool SM, int NW>
+__device__ __forceinline__ void level_candidates(Search<NW>& s)
+{
+    const Row<NW> r = Tab<SM, NW>::row(s, s.row);
+    s.entries = r.entries;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) s.R[w] = r.m[w] & s.A[w];
+    if (static_cast<int64_t>(r.m[NW - 1]) < 0) only_tried<NW>(s.tb + r.clears, s.R);
+}
+
+// whether the trials of the candidates r of a row have to be replayed
+template <int NW>
+__device__ __forceinline__ bool flagged(const Row<NW>& row, const uint64_t* r)
+{
+    return static_cast<int64_t>(row.m[NW - 1]) < 0 && (NW > 1 || (r[0] & (r[0] - 1)) != 0);
+}
+
+// of those, the ones above a slot
+template <int NW>
+__device__ __forceinline__ void above_slot(uint64_t* r, uint32_t slot, uint64_t above)
+{
+    if (NW == 1) {
+        r[0] &= above;
+    } else {
+#pragma unroll
+        for (int w = 0; w < NW; ++w)
+            r[w] = w < static_cast<int>(slot >> 6) ? 0ull : (w == static_cast<int>(slot >> 6) ? r[w] & above : r[w]);
+    }
+}
+
+// transition (kind_index << 2 | orientation) of a stack word
+template <bool SM, int NW>
+__device__ __forceinline__ uint32_t word_transition(const Search<NW>& s, uint32_t word)
+{
+    const uint32_t slot = word_slot(word), space = word_space(word);
+    const uint32_t* tb = s.tb;
+    uint32_t ki = __ldg(reinterpret_cast<const uint8_t*>(tb + __ldg(tb + 9)) + space * 64 * NW + slot);
+    const uint32_t nborder = __ldg(tb + 11);
+    if (space && ki >= nborder) ki -= nborder;
+    return (ki << 2) | (Tab<SM, NW>::entry(s, Tab<SM, NW>::row(s, word_row(word)).entries, slot) >> 14);
+}
+
+// (The functions below that are not inlined take the state by value: a reference would keep
+// the state of the whole kernel in local memory.)
+
+template <bool SM, int NW>
+__device__ __forceinline__ void start_puzzle(const BtLaunch& P, Search<NW>& s, uint32_t pz)
+{
+    s.pz = pz;
+    s.tb = P.ctables + P.coffset[pz];
+    s.n = SM ? P.chdr.n : __ldg(s.tb + 1);
+    s.space = 0;
+}
+
+template <int NW>
+__device__ __forceinline__ void start_search(Search<NW>& s, uint32_t len)
+{
+    s.L = len;
+    s.base = len;
+    s.nodes = 0;
+    s.sols = 0;
+    s.steps = 0;
+    s.active = true;
+}
+
+// no work: an empty set at the base level
+template <int NW>
+__device__ __forceinline__ void idle(Search<NW>& s)
+{
+    s.active = false;
+    s.L = 0;
+    s.base = 0;
+    s.nodes = 0;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) s.R[w] = 0;
+}
+
+// Starts an item of an earlier round: level `len` of a handed-back state, after the piece
+// placed there (or from the state's first slot when it is the state's own level).
+template <bool SM, int NW, int T>
+__device__ __forceinline__ void load_item(const BtLaunch& P, Search<NW>& s, const uint32_t* st, uint32_t len,
+                                          uint32_t* stk)
+{
+    const uint4 h = *reinterpret_cast<const uint4*>(st), g = *reinterpret_cast<const uint4*>(st + 4);
+    s.orig = static_cast<uint64_t>(h.x) | (static_cast<uint64_t>(h.y) << 32);
+    start_puzzle<SM, NW>(P, s, h.w);
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+        s.A[w] = *reinterpret_cast<const uint64_t*>(st + 8 + 2 * w);
+        s.O[w] = w ? 0ull : g.z | static_cast<uint64_t>(g.w) << 32;
+    }
+    s.row = static_cast<int>(g.x);
+    SlotBits bits{0ull, 0ull};
+    uint32_t from = 0;               // the slot placed at the level
+    const bool resumed = len < h.z;  // else the state's own level, from its first slot left
+    const uint32_t* pre = st + state_header(NW);
+    for (uint32_t l = 0; l < h.z; l += 4) {
+        const uint4 v = *reinterpret_cast<const uint4*>(pre + l);
+        const uint32_t word[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) {
+            if (l + j < len) {
+                stk[(l + j) * T] = word[j];
+            } else if (l + j < h.z) {
+                // a piece at or past the level is given back
+                const uint32_t slot = word_slot(word[j]);
+                const SlotBits q = Tab<SM, NW>::slot(P, s, word_space(word[j]), slot);
+                to_space<NW>(s, word_space(word[j]));
+                toggle<NW>(s.A, slot, q.toggle);
+                if (l + j == len) {
+                    s.row = word_row(word[j]);
+                    from = slot;
+                    bits = q;
+                }
+            }
+        }
+    }
+    to_space<NW>(s, desc_space(Tab<SM, NW>::desc(s, len)));
+    level_candidates<SM, NW>(s);
+    if (resumed) {
+        above_slot<NW>(s.R, from, bits.above);
+    } else if (g.y) {
+        above_slot<NW>(s.R, g.y - 1, Tab<SM, NW>::slot(P, s, s.space, g.y - 1).above);
+    }
+    start_search<NW>(s, len);
+}
+
+// Starts an initial record: a prefix of transitions from the expansion, or a level of a resumed
+// search with the transition it starts from.
+template <bool SM, int NW, int T>
+__device__ __forceinline__ void load_record(const BtLaunch& P, Search<NW>& s, const uint32_t* rec, uint32_t* stk)
+{
+    s.orig = static_cast<uint64_t>(rec[0]) | (static_cast<uint64_t>(rec[1]) << 32);
+    const uint32_t len = rec[2] & 0xFFFFu, start = rec[2] >> 16;
+    start_puzzle<SM, NW>(P, s, rec[3] & 0xFFFFu);
+    const uint32_t init = __ldg(s.tb + 8), nborder = __ldg(s.tb + 11);
+    const uint32_t width = SM ? P.chdr.width : __ldg(s.tb + 2);
+    const uint8_t* first = reinterpret_cast<const uint8_t*>(s.tb + __ldg(s.tb + 10));
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+        s.A[w] = ldg64(s.tb + init + 2 + 2 * w);
+        s.O[w] = w ? 0ull : ldg64(s.tb + init);
+    }
+    uint32_t west = 0;
+    for (uint32_t l = 0;; ++l) {
+        const uint4 d = Tab<SM, NW>::desc(s, l);
+        const uint32_t north = l ? stk[d.w * T] & 0xFFu : 0u;
+        s.row = row_at<NW>(d, west, north);
+        to_space<NW>(s, desc_space(d));
+        if (l == len) break;
+        const uint32_t t = (rec[4 + (l >> 1)] >> (16 * (l & 1))) & 0xFFFFu;
+        // corners follow the borders in space 1
+        const bool corner = l == 0 || l + 1 == width || l + width == s.n || l + 1 == s.n;
+        uint32_t slot = __ldg(first + 256 * s.space + (t >> 2) + (corner ? nborder : 0u));
+        const int entries = Tab<SM, NW>::row(s, s.row).entries;
+        uint32_t e = Tab<SM, NW>::entry(s, entries, slot);
+        // the piece's slots in this row ascend with the orientation
+        for (int k = 0; k < 3 && (e >> 14) != (t & 3u); ++k) e = Tab<SM, NW>::entry(s, entries, ++slot);
+        toggle<NW>(s.A, slot, Tab<SM, NW>::slot(P, s, s.space, slot).toggle);
+        stk[l * T] = make_word(e, slot, false, s.space, s.row);
+        west = e;
+    }
+    level_candidates<SM, NW>(s);
+    if (start) {
+        // a resumed level: drop the candidates below transition `start`
+        while (any<NW>(s.R)) {
+            const uint32_t slot = first_slot<NW>(s.R);
+            if (word_transition<SM, NW>(s, make_word(0, slot, false, s.space, s.row)) >= start) break;
+#pragma unroll
+            for (int w = 0; w < NW; ++w)
+                if (w == static_cast<int>(slot >> 6)) s.R[w] &= s.R[w] - 1;
+        }
+    }
+    start_search<NW>(s, len);
+}
+
+// Keeps the lexicographically smallest solution path of each puzzle, as record_solution of
+// emp_bt.cu does (bounded wait for the record's lock).
+template <bool SM, int NW, int T>
+__device__ __forceinline__ void record_solution(const BtLaunch& P, const Search<NW>& s, const uint32_t* stk)
+{
+    FirstRecord* r = P.first_records + s.pz;
+    atomicMin(&P.first_item[s.pz], (unsigned long long)s.orig);
+    if (s.orig > *(volatile unsigned long long*)&P.first_item[s.pz]) return;
+    const uint64_t give_up = global_ns() + P.first_lock_wait_ns;
+    while (atomicCAS(&r->lock, 0u, 1u) != 0u) {
+        if (global_ns() > give_up) {
+            atomicExch(&r->missed, 1u);
+            atomicOr(P.status, EMP_DEV_FIRST_LOST);
+            return;
+        }
+        __nanosleep(64);
+    }
+    __threadfence();
+    bool better = !r->has;
+    if (!better) {
+        for (uint32_t l = 0; l < s.n; ++l) {
+            const uint32_t mine = word_transition<SM, NW>(s, stk[l * T]), theirs = r->t[l];
+            if (mine != theirs) {
+                better = mine < theirs;
+                break;
+            }
+        }
+    }
+    if (better) {
+        for (uint32_t l = 0; l < s.n; ++l)
+            r->t[l] = static_cast<uint16_t>(word_transition<SM, NW>(s, stk[l * T]));
+        r->has = 1;
+    }
+    __threadfence();
+    atomicExch(&r->lock, 0u);
+}
+
+// A solution's whole path is on the stack (its last piece's word included).
+template <bool SM, int NW, int T>
+__device__ __noinline__ void solution_found(const BtLaunch& P, const Search<NW> s, const uint32_t* stk,
+                                            uint32_t placed)
+{
+    record_solution<SM, NW, T>(P, s, stk);
+    if (P.sols) {
+        const unsigned long long at = atomicAdd(P.sol_count, 1ull);
+        if (at < P.sol_capacity) {
+            SolutionRecord* r = P.sols + at;
+            r->orig = s.orig;
+            r->local = s.nodes + placed;
+            for (uint32_t l = 0; l < s.n; ++l)
+                r->t[l] = static_cast<uint16_t>(word_transition<SM, NW>(s, stk[l * T]));
+        }
+    }
+    if (P.stop_at_any) {
+        // first solution of the run: note the time and stop every thread
+        atomicCAS(&P.ctl->first_found_ns, 0ull, static_cast<unsigned long long>(global_ns()));
+        atomicExch(P.abort_flag, 1);
+    }
+}
+
+template <int NW>
+__device__ __forceinline__ void account(const BtLaunch& P, const Search<NW>& s)
+{
+    if (s.nodes) atomicAdd(&P.totals[2 * s.pz], (unsigned long long)s.nodes);
+    if (s.sols) atomicAdd(&P.totals[2 * s.pz + 1], (unsigned long long)s.sols);
+    if (P.item_nodes) {
+        if (s.nodes) atomicAdd(&P.item_nodes[s.orig], (unsigned long long)s.nodes);
+        if (s.sols) atomicAdd(&P.item_sols[s.orig], (unsigned long long)s.sols);
+    }
+}
+
+// Hands the remaining work of the thread to the next round: its state, in the slot that is this
+// thread's own, and one item per level that still holds candidates (the more bits say which).
+// Returns false when the item queue is full (the thread then keeps the work).
+template <bool SM, int NW, int T>
+__device__ __noinline__ bool split_state(const BtLaunch& P, uint32_t* out, const Search<NW> s, const uint32_t* stk)
+{
+    const bool here = any<NW>(s.R);
+    uint32_t cnt = here;
+    for (uint32_t l = s.base; l < s.L; ++l) cnt += word_more(stk[l * T]);
+    if (!cnt) return true;
+    unsigned long long* items = reinterpret_cast<unsigned long long*>(out + P.items_off);
+    unsigned long long k = atomicAdd(P.out_tail, (unsigned long long)cnt);
+    if (k + cnt > P.out_capacity) {
+        for (; cnt && k < P.out_capacity; ++k, --cnt) items[k] = kNoItem;  // reserved places that fit
+        return false;
+    }
+    const unsigned long long me = blockIdx.x * T + threadIdx.x;
+    for (uint32_t l = s.base; l < s.L; ++l)
+        if (word_more(stk[l * T])) items[k++] = (me << 32) | l;
+    if (here) items[k] = (me << 32) | s.L;
+    uint32_t* st = out + me * P.crec_words;
+    *reinterpret_cast<uint4*>(st) =
+        make_uint4(static_cast<uint32_t>(s.orig), static_cast<uint32_t>(s.orig >> 32), s.L, s.pz);
+    const uint64_t border = s.space ? s.A[0] : s.O[0];
+    *reinterpret_cast<uint4*>(st + 4) = make_uint4(static_cast<uint32_t>(s.row), here ? first_slot<NW>(s.R) : 0u,
+                                                   static_cast<uint32_t>(border), static_cast<uint32_t>(border >> 32));
+#pragma unroll
+    for (int w = 0; w < NW; ++w) *reinterpret_cast<uint64_t*>(st + 8 + 2 * w) = s.space ? s.O[w] : s.A[w];
+    uint32_t* pre = st + state_header(NW);
+    for (uint32_t l = 0; l < s.L; l += 4)  // the stack column holds a multiple of 4 levels
+        *reinterpret_cast<uint4*>(pre + l) =
+            make_uint4(stk[l * T], stk[(l + 1) * T], stk[(l + 2) * T], stk[(l + 3) * T]);
+    return true;
+}
+
+// Persistent search over the records of a round; the fetch, the hand-back rule and the
+// checks of the deadline, cancellation and stop-at-first flags are those of dfs_kernel.
+template <int NW, bool SM, bool GS, int T, int kStepsPerFetch>
+__global__ void __launch_bounds__(T, (NW == 1 && SM ? 768 : 512) / T) dfs_compact_kernel(const __grid_constant__ BtLaunch P)
+{
+    using TB = Tab<SM, NW>;
+    const uint32_t tid = threadIdx.x, lane = tid & 31;
+    if (SM) {
+        const uint4* src = reinterpret_cast<const uint4*>(P.ctables + P.coffset[0]);
+        uint4* dst = reinterpret_cast<uint4*>(g_smem);
+        for (uint32_t i = tid; i < P.smem_tab_words / 4; i += T) dst[i] = __ldg(src + i);
+        __syncthreads();
+    }
+    uint32_t* const stk = GS ? P.stack + (size_t)blockIdx.x * T * P.stack_levels + tid : g_smem + P.smem_tab_words + tid;
+    Search<NW> s;
+    idle<NW>(s);
+    bool fix = false;          // the level's candidates still hold what its row's trials remove
+    bool alive = true;
+    bool drained = false;      // warp-uniform: the input queue of this round is empty
+    uint32_t iteration = 0;    // warp-uniform loop counter
+    uint32_t since_check = 0;  // steps since the last look at the global flags
+    const uint64_t deadline = *(volatile unsigned long long*)&P.ctl->deadline;
+    const uint64_t n_in = P.n_in_from_ctl ? *(volatile unsigned long long*)&P.ctl->n_in : P.n_in;
+    // rounds after the first read what the one before handed back; in graph runs the two
+    // queues change roles every round
+    const uint32_t* in = P.in_rec;
+    uint32_t* out = P.out_rec;
+    if (P.swap_rec) {
+        if (*(volatile unsigned long long*)&P.ctl->rounds & 1ull) {
+            in = P.out_rec;
+            out = P.swap_rec;
+        } else {
+            in = P.swap_rec;
+        }
+    }
+    const unsigned long long* items =
+        P.in_items ? reinterpret_cast<const unsigned long long*>(in + P.items_off) : nullptr;
+    const uint32_t lt_mask = (1u << lane) - 1u;
+
+    for (;; ++iteration) {
+        // ---- work fetch: one atomic per warp, ranks from the ballot ----
+        const bool need = alive && !s.active;
+        const unsigned needmask = __ballot_sync(kFull, need);
+        if (needmask) {
+            const uint32_t leader = __ffs(needmask) - 1;
+            unsigned long long base = 0;
+            if (lane == leader) base = atomicAdd(P.cursor, (unsigned long long)__popc(needmask));
+            base = __shfl_sync(kFull, base, leader);
+            if (base + __popc(needmask) >= n_in) drained = true;
+            if (need) {
+                const uint64_t my = base + __popc(needmask & lt_mask);
+                if (my < n_in) {
+                    const unsigned long long item = items ? items[my] : 0ull;
+                    const uint32_t* rec = in + (items ? (item >> 32) : my) * (items ? P.crec_words : P.rec_words);
+                    if (items ? item != kNoItem : !(rec[3] & kEmptyRec)) {
+                        if (*(volatile int*)P.abort_flag) {
+                            P.incomplete[rec[3] & 0xFFFFu] = 1u;  // stopped: the work stays unsearched
+                        } else {
+                            if (items) load_item<SM, NW, T>(P, s, rec, static_cast<uint32_t>(item), stk);
+                            else load_record<SM, NW, T>(P, s, rec, stk);
+                            if (P.stop_at_first && s.orig > *(volatile unsigned long long*)&P.first_item[s.pz])
+                                idle<NW>(s);  // a lower subtree of this puzzle holds a solution
+                        }
+                    }
+                } else {
+                    alive = false;
+                }
+            }
+        } else if (!drained && (iteration & 31u) == 31u) {
+            // every warp learns within 32 rounds of steps that the queue ran dry
+            unsigned long long c = 0;
+            if (lane == 0) c = *(volatile unsigned long long*)P.cursor;
+            c = __shfl_sync(kFull, c, 0);
+            drained = c >= n_in;
+        }
+        if (!__any_sync(kFull, alive)) break;
+
+        // ---- steps: a warp-uniform trip count; a lane without work has an empty set at its
+        // base level and sits them out ----
+        uint32_t placed = 0;
+        for (int step = 0; step < kStepsPerFetch; ++step) {
+            // (1) an exhausted level: up to the one before, whose piece is given back
+            uint32_t popped = 0;
+            if (!any<NW>(s.R) && s.L != s.base) {
+                --s.L;
+                const uint32_t word = stk[s.L * T], slot = word_slot(word);
+                const SlotBits bits = TB::slot(P, s, word_space(word), slot);
+                to_space<NW>(s, word_space(word));
+                toggle<NW>(s.A, slot, bits.toggle);
+                s.row = word_row(word);
+                const Row<NW> r = TB::row(s, s.row);
+                s.entries = r.entries;
+#pragma unroll
+                for (int w = 0; w < NW; ++w) s.R[w] = r.m[w] & s.A[w];
+                fix = flagged<NW>(r, s.R);
+                above_slot<NW>(s.R, slot, bits.above);
+                popped = slot + 1;
+            }
+            // the trials of flagged rows, of a level popped to or just entered
+            if (__any_sync(kFull, fix)) {
+                if (fix) {
+                    level_candidates<SM, NW>(s);
+                    if (popped) above_slot<NW>(s.R, popped - 1, TB::slot(P, s, s.space, popped - 1).above);
+                    fix = false;
+                }
+                __syncwarp();
+            }
+            // (2) the next candidate of the level, and what it leaves the next one
+            bool solved = false;
+            if (any<NW>(s.R)) {
+                const uint32_t slot = first_slot<NW>(s.R);
+#pragma unroll
+                for (int w = 0; w < NW; ++w)
+                    if (NW == 1 || w == static_cast<int>(slot >> 6)) s.R[w] &= s.R[w] - 1;
+                const uint4 d = TB::desc(s, s.L + 1);
+                const uint32_t e = TB::entry(s, s.entries, slot);
+                const uint64_t bits = TB::slot(P, s, s.space, slot).toggle;
+                const uint32_t north = *reinterpret_cast<const uint8_t*>(&stk[d.w * T]);
+                const int crow = row_at<NW>(d, e, north);
+                const bool same = desc_space(d) == s.space;
+                const Row<NW> r = TB::row(s, crow);
+                ++placed;
+                // this level's word, should the search go down
+                stk[s.L * T] = make_word(e, slot, any<NW>(s.R), s.space, s.row);
+                uint64_t a[NW], c[NW];
+#pragma unroll
+                for (int w = 0; w < NW; ++w) {
+                    a[w] = s.A[w] ^ (NW == 1 || w == static_cast<int>(slot >> 6) ? bits : 0ull);
+                    c[w] = r.m[w] & (same ? a[w] : s.O[w]);
+                }
+                solved = s.L == s.n - 1;  // level n has no candidate
+                // (3) down, when the next level has one
+                if (any<NW>(c)) {
+                    fix = flagged<NW>(r, c);
+#pragma unroll
+                    for (int w = 0; w < NW; ++w) {
+                        const uint64_t o = s.O[w];
+                        s.A[w] = same ? a[w] : o;
+                        s.O[w] = same ? o : a[w];
+                        s.R[w] = c[w];
+                    }
+                    s.space = same ? s.space : s.space ^ 1u;
+                    ++s.L;
+                    s.row = crow;
+                    s.entries = r.entries;
+                }
+            }
+            if (__any_sync(kFull, solved)) {
+                if (solved) {
+                    ++s.sols;
+                    solution_found<SM, NW, T>(P, s, stk, placed);
+                }
+                __syncwarp();
+            }
+        }
+        s.nodes += placed;
+        if (s.active && !any<NW>(s.R) && s.L == s.base) {
+            account<NW>(P, s);
+            idle<NW>(s);
+        }
+        if (!s.active) continue;
+        s.steps += kStepsPerFetch;
+        since_check += kStepsPerFetch;
+
+        // ---- once the queue is empty, hand work back for the next round ----
+        if (drained && P.item_budget && s.steps >= P.item_budget) {
+            if (split_state<SM, NW, T>(P, out, s, stk)) {
+                account<NW>(P, s);
+                idle<NW>(s);
+                alive = false;
+                continue;
+            }
+            s.steps = 0;
+        }
+        // ---- deadline, cancellation and stop-at-first, every 4096 steps ----
+        if (since_check >= 4096) {
+            since_check = 0;
+            bool stop = *(volatile int*)P.abort_flag != 0;
+            if (deadline && global_ns() > deadline) {
+                stop = true;
+                atomicOr(P.status, EMP_DEV_TIMEOUT);
+            }
+            const bool superseded =
+                P.stop_at_first && s.orig > *(volatile unsigned long long*)&P.first_item[s.pz];
+            if (superseded || stop) {
+                account<NW>(P, s);
+                if (stop) {
+                    // the lane stays alive: it goes on taking records only to mark
+                    // their puzzles incomplete, so every dropped piece of work is known
+                    P.incomplete[s.pz] = 1u;
+                    atomicExch(P.abort_flag, 1);
+                    atomicOr(P.status, EMP_DEV_ABORTED);
+                } else {
+                    atomicOr(P.status, EMP_DEV_SUPERSEDED);
+                }
+                idle<NW>(s);
+            }
+        }
+    }
+}
+
+constexpr int kSteps = 32;
+
+template <int NW, int T>
+const void* symbol_t(bool sm, bool gs)
+{
+    if (sm) return gs ? reinterpret_cast<const void*>(&dfs_compact_kernel<NW, true, true, T, kSteps>)
+                      : reinterpret_cast<const void*>(&dfs_compact_kernel<NW, true, false, T, kSteps>);
+    return gs ? reinterpret_cast<const void*>(&dfs_compact_kernel<NW, false, true, T, kSteps>)
+              : reinterpret_cast<const void*>(&dfs_compact_kernel<NW, false, false, T, kSteps>);
+}
+
+template <int T>
+const void* symbol_nw(uint32_t nw, bool sm, bool gs)
+{
+    switch (nw) {
+        case 1: return symbol_t<1, T>(sm, gs);
+        case 2: return symbol_t<2, T>(sm, gs);
+        case 4: return symbol_t<4, T>(sm, gs);
+        default: return nullptr;
+    }
+}
+
+}  // namespace
+
+const void* compact_kernel_symbol(uint32_t nw, bool smem_tables, bool global_stack, uint32_t threads)
+{
+    switch (threads) {
+        case 128: return symbol_nw<128>(nw, smem_tables, global_stack);
+        case 256: return symbol_nw<256>(nw, smem_tables, global_stack);
+        case 512: return symbol_nw<512>(nw, smem_tables, global_stack);
+        default: return nullptr;
+    }
+}
+
+uint32_t compact_state_words(uint32_t max_levels, uint32_t nw)
+{
+    return state_header(nw) + compact_stack_levels(max_levels);
+}
+
+uint32_t compact_stack_levels(uint32_t max_levels) { return (max_levels + 3) & ~3u; }
+
+size_t compact_smem_bytes(uint32_t max_levels, uint32_t threads, uint32_t tab_words, bool global_stack)
+{
+    return sizeof(uint32_t) * (static_cast<size_t>(tab_words) +
+                               (global_stack ? 0 : static_cast<size_t>(compact_stack_levels(max_levels)) * threads));
+}
+
+cudaError_t launch_dfs_compact(const BtLaunch& P, uint32_t blocks, uint32_t threads, cudaStream_t stream)
+{
+    const bool gs = P.stack != nullptr;
+    const void* fn = compact_kernel_symbol(P.chdr.nw, P.smem_tab_words != 0, gs, threads);
+    if (!fn) return cudaErrorInvalidValue;
+    const size_t smem = compact_smem_bytes(P.max_levels, threads, P.smem_tab_words, gs);
+    void* args[] = {const_cast<BtLaunch*>(&P)};
+    return cudaLaunchKernel(fn, dim3(blocks), dim3(threads), args, smem, stream);
+}
+
+}  // namespace emp

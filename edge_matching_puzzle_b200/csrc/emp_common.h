@@ -2,6 +2,7 @@
 #pragma once
 
 #include "emp_b200.h"
+#include "emp_compact.h"
 #include "emp_model.h"
 
 #include <cuda_runtime.h>
@@ -64,6 +65,7 @@ struct emp_puzzle_t {
     std::vector<uint32_t> order;
     std::vector<emp::LevelPlan> plan;
     emp::DeviceTables tables;
+    std::vector<uint32_t> compact;  // compact search tables; empty when the puzzle has none
     uint32_t extra_count = 0;
 };
 

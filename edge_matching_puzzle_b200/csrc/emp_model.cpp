@@ -319,6 +319,9 @@ void build_device_tables(const PuzzleModel& m, const std::vector<LevelPlan>& pla
         align(b, 2);
         t.tinfo_off[k] = static_cast<uint32_t>(b.size());
         const uint32_t bits = 4 * m.nb_kind(k);
+        std::vector<uint32_t> allowed(m.kind_words[k], 0);
+        for (uint32_t e = 0; e < bits; ++e)
+            if (m.allowed(m.members[k][e >> 2], e & 3)) set_bit(allowed.data(), e);
         for (uint32_t e = 0; e < bits; ++e) {
             const uint32_t p = m.members[k][e >> 2], o = e & 3;
             uint32_t v = 0;
@@ -326,13 +329,10 @@ void build_device_tables(const PuzzleModel& m, const std::vector<LevelPlan>& pla
             // extra clears: bits the identical mask removes besides e itself,
             // restricted to allowed candidates (others never appear in a set)
             const uint32_t* im = &m.idmask[k][static_cast<size_t>(e) * m.kind_words[k]];
-            for (uint32_t e2 = 0; e2 < bits; ++e2) {
-                if (e2 == e || !m.allowed(m.members[k][e2 >> 2], e2 & 3)) continue;
-                if (!((im[e2 >> 5] >> (e2 & 31)) & 1u)) {
-                    v |= 1u << 20;
-                    break;
-                }
-            }
+            uint32_t extra = 0;
+            for (uint32_t w = 0; w < m.kind_words[k]; ++w)
+                extra |= ~im[w] & allowed[w] & ~(w == (e >> 5) ? 1u << (e & 31) : 0u);
+            if (extra) v |= 1u << 20;
             b.push_back(v);
         }
     }
@@ -349,13 +349,9 @@ void build_device_tables(const PuzzleModel& m, const std::vector<LevelPlan>& pla
         for (uint32_t e = 0; e < bits; ++e) {
             const uint32_t* im = &m.idmask[k][static_cast<size_t>(e) * m.kind_words[k]];
             for (uint32_t w = 0; w < t.kw[k]; ++w) {
-                uint64_t v = 0;
-                for (uint32_t i = 0; i < 64; ++i) {
-                    const uint32_t bit = 64 * w + i;
-                    // bits past the kind's candidates stay 1, like the reference's all-ones init
-                    const bool one = bit >= bits || ((im[bit >> 5] >> (bit & 31)) & 1u);
-                    if (one) v |= uint64_t(1) << i;
-                }
+                // bits past the kind's candidates stay 1, like the reference's all-ones init
+                uint64_t v = im[2 * w] | static_cast<uint64_t>(2 * w + 1 < m.kind_words[k] ? im[2 * w + 1] : 0u) << 32;
+                if (bits - 64 * w < 64) v |= ~uint64_t(0) << (bits - 64 * w);
                 push64(b, v);
             }
         }

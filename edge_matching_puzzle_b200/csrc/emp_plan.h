@@ -26,6 +26,10 @@ struct emp_bt_plan_t {
     DeviceBuffer totals, first_item, records, flags, item_nodes, item_sols, spill, prefix_out;
     DeviceBuffer stack;                       // kStackGlobal32: the threads' DFS stacks
     int stack_mode = emp::kStackShared32;
+    bool compact = false;                     // compact search (emp_btc.cu)
+    DeviceBuffer ctables, coff;
+    emp::CompactHeader chdr{};
+    uint32_t queue_words = 0;                 // words per record (compact: per state) of the round queues
     DeviceBuffer ctl, incomplete, puzzle_depth_dev;
     std::vector<uint32_t> puzzle_depth;       // per puzzle split depth
     bool adaptive = false;                    // per puzzle split depths (split_subtrees)
@@ -74,6 +78,11 @@ struct emp_bt_plan_t {
         if (evr1) cudaEventDestroy(evr1);
     }
 
+    cudaError_t launch_round(const emp::BtLaunch& P, cudaStream_t st) const
+    {
+        return compact ? emp::launch_dfs_compact(P, blocks, threads, st) : emp::launch_dfs(P, blocks, threads, st);
+    }
+
     emp::BtLaunch launch() const
     {
         emp::BtLaunch P;
@@ -111,6 +120,12 @@ struct emp_bt_plan_t {
         P.first_lock_init = cfg.hold_first_lock ? 1u : 0u;
         P.stack_mode = stack_mode;
         P.stack = stack.as<uint32_t>();
+        P.ctables = ctables.as<uint32_t>();
+        P.coffset = coff.as<uint64_t>();
+        P.chdr = chdr;
+        P.crec_words = queue_words;
+        P.items_off = static_cast<uint64_t>(queue_words) * blocks * threads;
+        P.stack_levels = emp::compact_stack_levels(max_levels);
         return P;
     }
 };
