@@ -149,9 +149,9 @@ emp_status expand(emp_bt_plan_t& pl)
     }
     uint32_t level = 0;
     for (; level < levels; ++level) {
-        CUDA_TRY(counts.alloc(sizeof(uint32_t) * std::max<uint64_t>(np, 1)));
-        CUDA_TRY(offsets.alloc(sizeof(uint64_t) * std::max<uint64_t>(np, 1)));
-        CUDA_TRY(bsums.alloc(sizeof(uint64_t) * emp::scan_block_sum_words(np)));
+        CUDA_TRY(counts.reserve(sizeof(uint32_t) * std::max<uint64_t>(np, 1)));
+        CUDA_TRY(offsets.reserve(sizeof(uint64_t) * std::max<uint64_t>(np, 1)));
+        CUDA_TRY(bsums.reserve(sizeof(uint64_t) * emp::scan_block_sum_words(np)));
         const uint8_t* fz = pl.adaptive ? frozen_dev.as<uint8_t>() : nullptr;
         CUDA_TRY(emp::launch_expand_frozen(L, parents.as<uint16_t>(), parent_puzzle.as<uint32_t>(), np, level,
                                            counts.as<uint32_t>(), nullptr, nullptr, nullptr, lnodes, lnodes + P, 0,
@@ -161,8 +161,8 @@ emp_status expand(emp_bt_plan_t& pl)
         uint64_t total = 0;
         CUDA_TRY(cudaMemcpyAsync(&total, grand.p, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
         CUDA_TRY(cudaStreamSynchronize(st));
-        CUDA_TRY(children.alloc(sizeof(uint16_t) * std::max<uint64_t>(total, 1) * (level + 1)));
-        CUDA_TRY(child_puzzle.alloc(sizeof(uint32_t) * std::max<uint64_t>(total, 1)));
+        CUDA_TRY(children.reserve(sizeof(uint16_t) * std::max<uint64_t>(total, 1) * (level + 1)));
+        CUDA_TRY(child_puzzle.reserve(sizeof(uint32_t) * std::max<uint64_t>(total, 1)));
         CUDA_TRY(emp::launch_expand_frozen(L, parents.as<uint16_t>(), parent_puzzle.as<uint32_t>(), np, level,
                                            counts.as<uint32_t>(), offsets.as<uint64_t>(), children.as<uint16_t>(),
                                            child_puzzle.as<uint32_t>(), lnodes, lnodes + P, 1, fz, st));
@@ -462,8 +462,9 @@ emp_status create_plan(const emp_puzzle* puzzles, uint32_t count, const emp_bt_c
     if (pl->cfg.table_placement == 2 && !pl->smem_tab_words)
         return fail(EMP_ERR_UNSUPPORTED, "tables can only be staged in shared memory for a single puzzle up to 64 KB");
     // launch geometry: the block size with the most resident warps per SM
-    cudaDeviceProp prop;
-    CUDA_TRY(cudaGetDeviceProperties(&prop, pl->device));
+    int sms = 0, smem_optin = 0;
+    CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, pl->device));
+    CUDA_TRY(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, pl->device));
     // default of the bitfield search: the shared 32-bit stack next to staged tables (a single
     // puzzle) while it leaves at least 16 warps per SM, else the global stack.  Measured on a
     // B200: 12x12 (8 warps per SM shared) 1.8e10 against 2.3e10.  The compact search (one word a
@@ -488,11 +489,11 @@ emp_status create_plan(const emp_puzzle* puzzles, uint32_t count, const emp_bt_c
                 pl->compact
                     ? emp::compact_smem_bytes(pl->max_levels, threads, pl->smem_tab_words, gs)
                     : emp::dfs_smem_bytes(pl->max_levels, pl->max_avail, threads, pl->smem_tab_words, pl->stack_mode);
-            if (smem > static_cast<size_t>(prop.sharedMemPerBlockOptin)) continue;
+            if (smem > static_cast<size_t>(smem_optin)) continue;
             // (the compact kernel's limit and carve-out are the same for every plan, so that a plan
             // created later never lowers them under an earlier one)
             CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          static_cast<int>(pl->compact ? prop.sharedMemPerBlockOptin : smem)));
+                                          pl->compact ? smem_optin : static_cast<int>(smem)));
             if (pl->compact && !gs && !pl->smem_tab_words)
                 CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 44));
             int per_sm = 0;
@@ -507,7 +508,7 @@ emp_status create_plan(const emp_puzzle* puzzles, uint32_t count, const emp_bt_c
             if (per_sm >= 1 && warps > best_warps) {
                 best_warps = warps;
                 pl->threads = threads;
-                pl->blocks = static_cast<uint32_t>(per_sm) * static_cast<uint32_t>(prop.multiProcessorCount);
+                pl->blocks = static_cast<uint32_t>(per_sm) * static_cast<uint32_t>(sms);
             }
         }
         return EMP_OK;
@@ -521,6 +522,8 @@ emp_status create_plan(const emp_puzzle* puzzles, uint32_t count, const emp_bt_c
         return fail(EMP_ERR_UNSUPPORTED, "per-thread DFS state does not fit shared memory; use fewer threads per block");
     const uint64_t resident = static_cast<uint64_t>(pl->blocks) * pl->threads;
     if (pl->compact) {
+        // initial records hold a header and the prefix alone (a 10x10 board has 6.3 million of them)
+        if (!resume) pl->rec_words = 4 + (pl->depth + 1) / 2;
         if (pl->stack_mode == emp::kStackGlobal32)
             CUDA_TRY(pl->stack.alloc(sizeof(uint32_t) * resident * emp::compact_stack_levels(pl->max_levels)));
         // round queues: a thread hands its state back at most once a round, with an item per

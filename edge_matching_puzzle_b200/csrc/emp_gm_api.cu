@@ -94,9 +94,10 @@ extern "C" emp_status emp_glutton_max(emp_puzzle puzzle, const emp_gm_config* co
     const emp::PuzzleModel& m = puzzle->model;
     int dev = 0;
     EMP_TRY(emp::select_device(cfg.device, &dev));
-    cudaDeviceProp prop;
-    CUDA_TRY(cudaGetDeviceProperties(&prop, dev));
-    if (emp::gm_smem_bytes() > static_cast<size_t>(prop.sharedMemPerBlockOptin))
+    int sms = 0, smem_optin = 0;
+    CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    CUDA_TRY(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    if (emp::gm_smem_bytes() > static_cast<size_t>(smem_optin))
         return fail(EMP_ERR_UNSUPPORTED, "glutton max level state does not fit shared memory");
     const uint32_t S = m.n;
     std::vector<uint8_t> pieces(256 * 4, 0);
@@ -117,8 +118,8 @@ extern "C" emp_status emp_glutton_max(emp_puzzle puzzle, const emp_gm_config* co
     DeviceBuffer d_pieces, d_cc, d_infos, d_state, d_grid;
     const size_t tri = static_cast<size_t>(S) * (S + 1) / 2;
     uint32_t blocks = cfg.blocks;
-    if (!blocks) blocks = static_cast<uint32_t>(prop.multiProcessorCount);
-    blocks = std::min<uint32_t>(blocks, std::min<uint32_t>(emp::kMaxGridBlocks, prop.multiProcessorCount));
+    if (!blocks) blocks = static_cast<uint32_t>(sms);
+    blocks = std::min<uint32_t>(blocks, std::min<uint32_t>(emp::kMaxGridBlocks, sms));
     if (blocks > 1) {
         CUDA_TRY(d_grid.alloc(sizeof(emp::GmGrid)));
         CUDA_TRY(cudaMemset(d_grid.p, 0, sizeof(emp::GmGrid)));
@@ -224,9 +225,9 @@ extern "C" emp_status emp_glutton_max_noalloc(emp_puzzle puzzle, const emp_gm_co
                                              std::to_string(kNoAllocMaxColours));
     int dev = 0;
     EMP_TRY(emp::select_device(cfg.device, &dev));
-    cudaDeviceProp prop;
-    CUDA_TRY(cudaGetDeviceProperties(&prop, dev));
-    if (emp::gm_smem_bytes() > static_cast<size_t>(prop.sharedMemPerBlockOptin))
+    int smem_optin = 0;
+    CUDA_TRY(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    if (emp::gm_smem_bytes() > static_cast<size_t>(smem_optin))
         return fail(EMP_ERR_UNSUPPORTED, "glutton max level state does not fit shared memory");
 
     // The device address of the scratch array on the current device, looked up on

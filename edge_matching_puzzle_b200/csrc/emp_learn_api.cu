@@ -484,7 +484,7 @@ extern "C" emp_status emp_bt_plan_order(emp_bt_plan plan, emp_mlp model)
     FeatTables ft;
     EMP_TRY(ft.upload(plan->puzzles));
     const uint32_t per = depth - 1;
-    const uint64_t chunk = std::max<uint64_t>(1, (1ull << 21) / per);  // 2M feature rows (2 GB of bf16) at most
+    const uint64_t chunk = std::max<uint64_t>(1, (1ull << 16) / per);  // 65536 feature rows: 64 MB, which stay in L2
     DeviceBuffer d_rank, d_score, d_items, d_x, d_s, d_err;
     CUDA_TRY(d_rank.alloc(4ull * P));
     CUDA_TRY(cudaMemcpy(d_rank.p, rank.data(), 4ull * P, cudaMemcpyHostToDevice));
