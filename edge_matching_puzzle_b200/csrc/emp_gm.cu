@@ -13,18 +13,27 @@
 //      push, apply the colour constraints of its sides;
 // popping when a level fails (CUDA_glutton_max_stack.h:437-522).
 //
-// B200 design: one 1024-thread block per search keeps the level in shared
-// memory together with per-level statistics -- nibble counts N[j][q] of piece
-// q at free position j, bit totals A[j], per-piece sums S[q] and, per piece,
-// the six smallest and six largest A[j]-N[j][q].  A trial then only scans the
-// (at most four) colour-constrained neighbour positions word by word; every
-// other position contributes A[j]-N[j][p] and the piece counts follow from
-// S[q]-N[i][q] minus what the neighbours lost.  This gives the reference's
-// (valid, total, min, max) exactly at a fraction of its cost.  Step 1 runs as
-// Jacobi passes (all candidates against the same level, then all removals):
-// validity only gets harder as bits disappear, so the passes reach the same
-// greatest fixpoint as the reference's in-place sweep, and they empty a
-// position exactly when the reference's sweep does.
+// B200 design: 1024-thread blocks keep the level in shared memory together with per-level
+// statistics -- orientation counts N[j][q] of piece q at free position j, bit totals A[j],
+// per-piece sums S[q] and, per piece, the six smallest and six largest A[j]-N[j][q].  A trial
+// then looks at the (at most four) colour-constrained neighbour positions alone; every other
+// position contributes A[j]-N[j][p], and the piece counts follow from S[q]-N[i][q] minus what
+// the neighbours lost.  This gives the reference's (valid, total, min, max) exactly.  Step 1
+// runs as Jacobi passes (all candidates against the same level, then all removals): validity
+// only gets harder as bits disappear, so the passes reach the same greatest fixpoint as the
+// reference's in-place sweep, and they empty a position exactly when the reference's sweep does.
+//
+// A trial is made by a group of G lanes, G the words that hold pieces (8, 16 or 32: up to 64,
+// 128, 256 pieces), lane w with word w, the pieces 8w..8w+7.  A trial's piece counts are eight
+// 16-bit numbers a lane: what position i and its neighbours leave of S (the same for every
+// candidate of i, kept in registers) plus what the neighbours keep, counted nibble by nibble
+// with bit operations.  The candidates of a pass are dealt out evenly by rank, so a group gets
+// a run of neighbouring candidates, nearly all of one position, and no work counter is needed.
+//
+// What bounds it: the trials' instructions and latency.  Measured on a B200, whole calls:
+// 16x16 (5/17 colours, 300 pushes, 148 blocks) 165 ms with a warp per word of candidates and
+// full scans for the lists, 42 ms now, 31 us a pass of 43 000 trials; 8x8 on one block (150
+// pushes) 162 ms, now 21 ms.
 #include "emp_gm.h"
 
 #include <cuda_runtime.h>
@@ -38,31 +47,30 @@ constexpr unsigned kFull = 0xFFFFFFFFu;
 constexpr uint64_t kBarrierWaitNs = 5000000000ull;  // 5 s: far beyond one validity pass
 
 struct GmSmem {
-    uint32_t X[256][32];       // infos of the current level
+    alignas(16) uint32_t X[256][32];       // infos of the current level
     uint32_t inval[256][32];   // candidates found invalid in this pass
-    uint8_t N[256][256];       // N[j][q]: orientations of piece q left at info j
+    alignas(16) uint8_t N[256][256];  // N[j][q]: orientations of piece q left at info j
     uint32_t lo[256][6];       // per piece q: six smallest (A[j]-N[j][q]) << 16 | j, ~0 empty
     uint32_t hi[256][6];       // per piece q: six largest (A[j]-N[j][q]+1) << 16 | j, 0 empty
-    uint32_t lo2[256][6];      // the same two lists over the second half of the infos,
-    uint32_t hi2[256][6];      // merged into lo / hi at the end of each statistics pass
-    uint16_t S2[256];
-    uint32_t partA[32];        // per warp: bits of its infos, and whether one is empty
-    uint32_t partE[32];
     uint32_t cc[32][4][32];    // colour constraints
+    alignas(16) uint32_t K[256];  // A[j] << 8 | j, ~0 past the last info
+    uint32_t cum[257];         // candidates of the infos before j
+    uint32_t part[16][64];     // partial sums of N, four pieces a word
     uint16_t A[256];           // bits of info j
-    uint16_t S[256];           // sum over j of N[j][q]
-    uint8_t pieces[256][4];
+    alignas(16) uint16_t S[256];  // sum over j of N[j][q]
+    uint16_t rank[4][256];     // partial ranks of K[j]
+    uint8_t ord[256];          // infos in ascending order of A
+    alignas(4) uint8_t pieces[256][4];
     uint32_t position_index[256];
     uint32_t info_index[256];
     uint32_t played[256];      // this block's copy of the played stack
     uint32_t avail[8];
     unsigned long long warp_key[32];
     uint32_t warp_order[32];
-    uint32_t warp_trials[32];
+    unsigned long long trials, pushes;  // of the whole search, counted alike by every block
     uint32_t sumA;
     uint32_t any_invalid;
     uint32_t any_empty;
-    uint32_t next_info;
     uint32_t best_order;       // chosen candidate: info << 10 | word << 5 | bit; ~0 none
     uint32_t level, new_level, pop_index, stop, apply_failed;
 };
@@ -77,22 +85,6 @@ __device__ __forceinline__ uint64_t global_ns()
     uint64_t t;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
     return t;
-}
-
-__device__ __forceinline__ uint32_t warp_sum(uint32_t v)
-{
-    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
-    return v;
-}
-__device__ __forceinline__ uint32_t warp_min(uint32_t v)
-{
-    for (int o = 16; o; o >>= 1) v = min(v, __shfl_xor_sync(kFull, v, o));
-    return v;
-}
-__device__ __forceinline__ uint32_t warp_max(uint32_t v)
-{
-    for (int o = 16; o; o >>= 1) v = max(v, __shfl_xor_sync(kFull, v, o));
-    return v;
 }
 
 // get_best_candidate's preference (include/CUDA_glutton_max.h:1196-1295): is candidate
@@ -119,107 +111,167 @@ __device__ __forceinline__ void warp_best(unsigned long long& k, uint32_t& o, bo
     }
 }
 
-__device__ __forceinline__ bool piece_available(const GmSmem& sm, uint32_t q)
+// orientation counts of the eight pieces of a word, in its nibbles
+__device__ __forceinline__ uint32_t nibble_counts(uint32_t v)
 {
-    return (sm.avail[q >> 5] >> (q & 31)) & 1u;
+    v -= (v >> 1) & 0x55555555u;
+    return (v & 0x33333333u) + ((v >> 2) & 0x33333333u);
 }
 
-// Six smallest (ASC) or largest of A[j]-N[j][q] over infos j in [j0, j1) for piece q,
-// as sorted lists of distinct keys (the info index in the low bits).
+// Keeps the six smallest (ASC) or largest keys.
 template <bool ASC>
-__device__ __forceinline__ void extreme_six(const GmSmem& sm, uint32_t q, uint32_t j0, uint32_t j1, uint32_t* best,
-                                            uint32_t* sum)
+__device__ __forceinline__ void keep_six(uint32_t* best, uint32_t v)
 {
-    uint32_t s = 0;
 #pragma unroll
-    for (int k = 0; k < 6; ++k) best[k] = ASC ? ~0u : 0u;
-    for (uint32_t j = j0; j < j1; ++j) {
-        const uint32_t n = sm.N[j][q];
-        s += n;
-        uint32_t v = ((sm.A[j] - n + (ASC ? 0u : 1u)) << 16) | j;
-#pragma unroll
-        for (int k = 0; k < 6; ++k) {
-            const uint32_t keep = ASC ? min(best[k], v) : max(best[k], v);
-            v = ASC ? max(best[k], v) : min(best[k], v);
-            best[k] = keep;
-        }
+    for (int k = 0; k < 6; ++k) {
+        const uint32_t keep = ASC ? min(best[k], v) : max(best[k], v);
+        v = ASC ? max(best[k], v) : min(best[k], v);
+        best[k] = keep;
     }
-    *sum = s;
 }
 
-// the first six of two sorted six-lists (ascending for ASC, else descending)
-template <bool ASC>
-__device__ __forceinline__ void merge_six(uint32_t* a, const uint32_t* b)
-{
-    uint32_t out[6];
-    int i = 0, k = 0;
-#pragma unroll
-    for (int o = 0; o < 6; ++o) {
-        const uint32_t x = a[i < 6 ? i : 5], y = b[k < 6 ? k : 5];
-        const bool take_a = k >= 6 || (i < 6 && (ASC ? x < y : x > y));
-        out[o] = take_a ? x : y;
-        i += take_a;
-        k += !take_a;
-    }
-#pragma unroll
-    for (int o = 0; o < 6; ++o) a[o] = out[o];
-}
-
-// Per-pass statistics of the current level (block-wide).  The per-piece scans run in
-// four groups of 256 threads (six smallest / six largest, each over one half of the
-// infos), merged afterwards; the lists are sets of distinct keys, so the halves and
-// the merge give the lists of one scan over all infos.
-__device__ void level_statistics(GmSmem& sm, uint32_t nb, uint32_t tid)
+// Per-pass statistics of the current level (block-wide).  The six smallest and largest
+// A[j]-N[j][q] of a piece are found by visiting the infos in order of A: N is at most 4, so
+// the visit ends once no later info can enter the list (a scan of all 256 infos for each
+// piece and list took most of the statistics' time).
+__device__ void level_statistics(GmSmem& sm, uint32_t n, uint32_t nb, uint32_t tid)
 {
     const uint32_t lane = tid & 31, warp = tid >> 5;
-    uint32_t asum = 0, aempty = 0;
-    for (uint32_t j = warp; j < nb; j += kThreads / 32) {
-        const uint32_t word = sm.X[j][lane];
-        uint32_t packed0 = 0, packed1 = 0;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            packed0 |= static_cast<uint32_t>(__popc((word >> (4 * k)) & 0xFu)) << (8 * k);
-            packed1 |= static_cast<uint32_t>(__popc((word >> (4 * (k + 4))) & 0xFu)) << (8 * k);
+    for (uint32_t j = warp; j < 256; j += kThreads / 32) {
+        uint32_t a = 0;
+        if (j < nb) {
+            const uint32_t word = sm.X[j][lane];
+            const uint32_t x = nibble_counts(word), even = x & 0x0F0F0F0Fu, odd = (x >> 4) & 0x0F0F0F0Fu;
+            *reinterpret_cast<uint2*>(&sm.N[j][8 * lane]) =
+                make_uint2(__byte_perm(even, odd, 0x5140), __byte_perm(even, odd, 0x7362));
+            a = __reduce_add_sync(kFull, __popc(word));
         }
-        reinterpret_cast<uint32_t*>(sm.N[j])[2 * lane] = packed0;
-        reinterpret_cast<uint32_t*>(sm.N[j])[2 * lane + 1] = packed1;
-        const uint32_t a = warp_sum(__popc(word));
-        if (lane == 0) sm.A[j] = static_cast<uint16_t>(a);
-        asum += a;
-        aempty |= a == 0;
-    }
-    if (lane == 0) {
-        sm.partA[warp] = asum;
-        sm.partE[warp] = aempty;
+        if (lane == 0) {
+            sm.A[j] = static_cast<uint16_t>(a);
+            sm.K[j] = j < nb ? (a << 8) | j : ~0u;
+        }
     }
     __syncthreads();
     {
-        const uint32_t q = tid & 255u, group = tid >> 8, half = nb / 2;
-        const uint32_t j0 = (group & 1u) ? half : 0u, j1 = (group & 1u) ? nb : half;
-        uint32_t best[6], s;
-        if (group < 2) extreme_six<true>(sm, q, j0, j1, best, &s);
-        else extreme_six<false>(sm, q, j0, j1, best, &s);
-        uint32_t* dst = group == 0 ? sm.lo[q] : group == 1 ? sm.lo2[q] : group == 2 ? sm.hi[q] : sm.hi2[q];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) dst[k] = best[k];
-        if (group == 0) sm.S[q] = static_cast<uint16_t>(s);
-        if (group == 1) sm.S2[q] = static_cast<uint16_t>(s);
+        // sums of N: four pieces a word, 16 infos a thread (at most 64 a byte)
+        const uint32_t col = tid & 63u, group = tid >> 6;
+        uint32_t acc = 0;
+        for (uint32_t j = group; j < nb; j += 16) acc += *reinterpret_cast<const uint32_t*>(&sm.N[j][4 * col]);
+        sm.part[group][col] = acc;
+        // ranks: 64 keys a thread
+        const uint32_t j = tid & 255u, from = 64 * (tid >> 8), mine = sm.K[j];
+        uint32_t before = 0;
+        if (from < nb) {
+#pragma unroll 4
+            for (uint32_t k = 0; k < 64; k += 4) {
+                const uint4 v = *reinterpret_cast<const uint4*>(&sm.K[from + k]);
+                before += (v.x < mine) + (v.y < mine) + (v.z < mine) + (v.w < mine);
+            }
+        }
+        sm.rank[tid >> 8][j] = static_cast<uint16_t>(before);
     }
     __syncthreads();
     if (tid < 256) {
-        merge_six<true>(sm.lo[tid], sm.lo2[tid]);
-        sm.S[tid] = static_cast<uint16_t>(sm.S[tid] + sm.S2[tid]);
+        uint32_t s = 0;
+        for (uint32_t g = 0; g < 16; ++g) s += (sm.part[g][tid >> 2] >> (8 * (tid & 3u))) & 0xFFu;
+        sm.S[tid] = static_cast<uint16_t>(s);
     } else if (tid < 512) {
-        merge_six<false>(sm.hi[tid - 256], sm.hi2[tid - 256]);
+        const uint32_t j = tid - 256;
+        if (j < nb) sm.ord[sm.rank[0][j] + sm.rank[1][j] + sm.rank[2][j] + sm.rank[3][j]] = static_cast<uint8_t>(j);
     } else if (tid < 544) {
-        const uint32_t a = warp_sum(sm.partA[lane]);
-        const uint32_t empty = __any_sync(kFull, sm.partE[lane] != 0);
-        if (lane == 0) {
-            sm.sumA = a;
+        uint32_t a[8], sum = 0;
+        bool empty = false;
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) {
+            const uint32_t j = 8 * lane + k;
+            a[k] = sum;
+            sum += sm.A[j];
+            empty |= j < nb && sm.A[j] == 0;
+        }
+        uint32_t x = sum;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(kFull, x, o);
+            if (lane >= static_cast<uint32_t>(o)) x += y;
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) sm.cum[8 * lane + k] = x - sum + a[k];
+        empty = __any_sync(kFull, empty);
+        if (lane == 31) {
+            sm.cum[256] = x;
+            sm.sumA = x;
             sm.any_empty = empty;
         }
     }
     __syncthreads();
+    if (tid < 512) {
+        const uint32_t q = tid & 255u;
+        uint32_t best[6];
+        if (q < n && sm.S[q]) {
+            if (tid < 256) {
+#pragma unroll
+                for (int k = 0; k < 6; ++k) best[k] = ~0u;
+                for (uint32_t t = 0; t < nb; ++t) {
+                    const uint32_t j = sm.ord[t], a = sm.A[j];
+                    if (a >= (best[5] >> 16) + 4) break;
+                    keep_six<true>(best, ((a - sm.N[j][q]) << 16) | j);
+                }
+#pragma unroll
+                for (int k = 0; k < 6; ++k) sm.lo[q][k] = best[k];
+            } else {
+#pragma unroll
+                for (int k = 0; k < 6; ++k) best[k] = 0u;
+                for (uint32_t t = nb; t-- > 0;) {
+                    const uint32_t j = sm.ord[t], a = sm.A[j];
+                    if (a + 1 <= (best[5] >> 16)) break;
+                    keep_six<false>(best, ((a - sm.N[j][q] + 1) << 16) | j);
+                }
+#pragma unroll
+                for (int k = 0; k < 6; ++k) sm.hi[q][k] = best[k];
+            }
+        }
+    }
+    __syncthreads();
+}
+
+// What the trials of one position share, in the registers of a group of G lanes.
+struct TrialSite {
+    uint32_t j[4];      // free neighbours by side (N, E, S, W); 0xFFFF none
+    uint32_t x[4];      // this lane's word of their infos, 0 for none
+    uint32_t left[4];   // 16-bit pairs: S[q] less this position's and the neighbours' N, of the
+                        // lane's pieces (0,2) (4,6) (1,3) (5,7)
+    uint32_t sum_a;     // bits of the other positions
+};
+
+template <int G>
+__device__ __forceinline__ void start_site(const GmSmem& sm, uint32_t nb, uint32_t i, uint32_t width, uint32_t height,
+                                           uint32_t lane, TrialSite& t)
+{
+    const uint32_t pos = sm.position_index[i], px = pos % width, py = pos / width;
+    const uint4 s8 = *reinterpret_cast<const uint4*>(&sm.S[8 * lane]);  // (0,1) (2,3) (4,5) (6,7)
+    const uint2 ni = *reinterpret_cast<const uint2*>(&sm.N[i][8 * lane]);
+    uint2 n = ni;  // bytes: at most 4 a position
+    t.sum_a = sm.sumA - sm.A[i];
+#pragma unroll
+    for (uint32_t s = 0; s < 4; ++s) {
+        const bool inside = s == 0 ? py > 0 : s == 1 ? px + 1 < width : s == 2 ? py + 1 < height : px > 0;
+        const uint32_t npos = s == 0 ? pos - width : s == 1 ? pos + 1 : s == 2 ? pos + width : pos - 1;
+        const uint32_t j = inside ? sm.info_index[npos] : ~0u;
+        const bool free = j < nb;
+        t.j[s] = free ? j : 0xFFFFu;
+        t.x[s] = 0;
+        if (free) {
+            t.x[s] = sm.X[j][lane];
+            const uint2 v = *reinterpret_cast<const uint2*>(&sm.N[j][8 * lane]);
+            n.x += v.x;
+            n.y += v.y;
+            t.sum_a -= sm.A[j];
+        }
+    }
+    // 16-bit pairs, no borrow between halves: S[q] counts every one of these positions
+    t.left[0] = __byte_perm(s8.x, s8.y, 0x5410) - __byte_perm(n.x, 0u, 0x4240);
+    t.left[1] = __byte_perm(s8.z, s8.w, 0x5410) - __byte_perm(n.y, 0u, 0x4240);
+    t.left[2] = __byte_perm(s8.x, s8.y, 0x7632) - __byte_perm(n.x, 0u, 0x4341);
+    t.left[3] = __byte_perm(s8.z, s8.w, 0x7632) - __byte_perm(n.y, 0u, 0x4341);
 }
 
 struct Trial {
@@ -227,99 +279,99 @@ struct Trial {
     uint32_t total, mn, mx;
 };
 
-// Trial placement of (info i, word wc, bit b) on the current level, warp-wide
-// (lane w owns word w, i.e. pieces 8w..8w+7).  Mirrors the lambdas of
-// remove_invalid_transitions and get_best_candidate.
-__device__ Trial trial(const GmSmem& sm, uint32_t nb, uint32_t i, uint32_t wc, uint32_t b, uint32_t width,
-                       uint32_t lane)
+template <int G>
+__device__ __forceinline__ uint32_t group_add(uint32_t v, uint32_t gmask)
+{
+    if (G == 32) return __reduce_add_sync(kFull, v);
+    for (int o = G / 2; o; o >>= 1) v += __shfl_xor_sync(gmask, v, o);
+    return v;
+}
+
+// Trial placement of (info i, word wc, bit b) on the current level by a group of lanes.  Mirrors
+// the lambdas of remove_invalid_transitions and get_best_candidate.  `taken`: 0xFFFF in the
+// 16-bit place of each piece of the lane that is not available (ordered as TrialSite::left).
+template <int G>
+__device__ __forceinline__ Trial trial(const GmSmem& sm, const TrialSite& t, const uint32_t* taken, uint32_t i,
+                                       uint32_t wc, uint32_t b, uint32_t lane, uint32_t gshift, uint32_t gmask)
 {
     Trial r{true, 0, ~0u, 0};
-    const uint32_t p = 8 * wc + b / 4, o = b & 3u;
-    const uint32_t pos = sm.position_index[i];
-    const uint32_t pm = lane == wc ? ~(0xFu << (4 * (b / 4))) : kFull;
-    const int off[4] = {-static_cast<int>(width), 1, static_cast<int>(width), -1};
-    uint32_t nj[4], ncnt[4];
-    uint32_t nn = 0;
+    const uint32_t k = b >> 2, p = 8 * wc + k;
+    const bool own = lane == wc;
+    const uint32_t pm = own ? ~(0xFu << (4 * k)) : kFull;
+    const uint32_t c4 = *reinterpret_cast<const uint32_t*>(sm.pieces[p]);
+    const uint32_t col = __funnelshift_r(c4, c4, 8 * (b & 3u));  // byte s: colour of side s
     // apply_color_constraints (CUDA_glutton_max.h:531-612)
-    for (uint32_t s = 0; s < 4; ++s) {
-        const uint32_t col = sm.pieces[p][(s + o) & 3u];
-        if (!col) continue;
-        const uint32_t npos = static_cast<uint32_t>(static_cast<int>(pos) + off[s]);
-        const uint32_t j = sm.info_index[npos];
-        if (j >= nb) continue;  // position not free
-        const uint32_t rw = sm.X[j][lane] & sm.cc[col - 1][s][lane] & pm;
-        const uint32_t pc = warp_sum(__popc(rw));
-        if (!pc) {
-            r.valid = false;
-            return r;
-        }
-        uint32_t packed = 0;
+    uint32_t even = 0, odd = 0, pc01 = 0, pc23 = 0;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) packed |= static_cast<uint32_t>(__popc((rw >> (4 * k)) & 0xFu)) << (3 * k);
-        nj[nn] = j;
-        ncnt[nn] = packed;
-        ++nn;
-        r.total += pc;
+    for (uint32_t s = 0; s < 4; ++s) {
+        const uint32_t c = (col >> (8 * s)) & 0xFFu;
+        uint32_t rw = 0;
+        if (c && t.j[s] != 0xFFFFu) rw = t.x[s] & sm.cc[c - 1][s][lane] & pm;
+        const uint32_t x = nibble_counts(rw);
+        even += x & 0x0F0F0F0Fu;
+        odd += (x >> 4) & 0x0F0F0F0Fu;
+        const uint32_t pc = __popc(rw);
+        if (s < 2) pc01 += pc << (16 * s);
+        else pc23 += pc << (16 * (s - 2));
+    }
+    pc01 = group_add<G>(pc01, gmask);
+    pc23 = group_add<G>(pc23, gmask);
+    uint32_t kept = 0;
+#pragma unroll
+    for (uint32_t s = 0; s < 4; ++s) {
+        if (t.j[s] == 0xFFFFu || !((col >> (8 * s)) & 0xFFu)) continue;
+        const uint32_t pc = ((s < 2 ? pc01 : pc23) >> (16 * (s & 1u))) & 0xFFFFu;
+        r.valid &= pc != 0;
+        kept += pc;
         r.mn = min(r.mn, pc);
         r.mx = max(r.mx, pc);
     }
-    // every other free position keeps X[j] without piece p (apply_simple_mask)
-    uint32_t sum_a = sm.sumA - sm.A[i];
-    uint32_t sum_n = sm.S[p] - sm.N[i][p];
-    for (uint32_t k = 0; k < nn; ++k) {
-        sum_a -= sm.A[nj[k]];
-        sum_n -= sm.N[nj[k]][p];
-    }
-    r.total += sum_a - sum_n;
-    auto excluded = [&](uint32_t j) {
-        bool e = j == i;
-        for (uint32_t k = 0; k < nn; ++k) e |= j == nj[k];
-        return e;
-    };
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-        const uint32_t e = sm.lo[p][k];
-        if (e == ~0u) break;
-        if (!excluded(e & 0xFFFFu)) {
-            const uint32_t v = e >> 16;
-            if (v == 0) {
-                r.valid = false;
-                return r;
-            }
-            r.mn = min(r.mn, v);
-            break;
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-        const uint32_t e = sm.hi[p][k];
-        if (e == 0u) break;
-        if (!excluded(e & 0xFFFFu)) {
-            r.mx = max(r.mx, (e >> 16) - 1u);
-            break;
-        }
-    }
     // pieces: every available piece other than p needs a place left
-    uint32_t psum = 0, pmin = ~0u, pmax = 0;
-    bool bad = false;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const uint32_t q = 8 * lane + k;
-        if (q == p || !piece_available(sm, q)) continue;
-        uint32_t c = static_cast<uint32_t>(sm.S[q]) - sm.N[i][q];
-        for (uint32_t kk = 0; kk < nn; ++kk) c -= sm.N[nj[kk]][q] - ((ncnt[kk] >> (3 * k)) & 7u);
-        bad |= c == 0;
-        psum += c;
-        pmin = min(pmin, c);
-        pmax = max(pmax, c);
+    const uint32_t c0 = t.left[0] + __byte_perm(even, 0u, 0x4140), c1 = t.left[1] + __byte_perm(even, 0u, 0x4342);
+    const uint32_t c2 = t.left[2] + __byte_perm(odd, 0u, 0x4140), c3 = t.left[3] + __byte_perm(odd, 0u, 0x4342);
+    const uint32_t at = own ? 0xFFFFu << (8 * (k & 2u)) : 0u;  // p's half
+    const uint32_t m0 = (k & 5u) == 0u ? at : 0u, m1 = (k & 5u) == 4u ? at : 0u;
+    const uint32_t m2 = (k & 5u) == 1u ? at : 0u, m3 = (k & 5u) == 5u ? at : 0u;
+    const uint32_t lo = __vminu2(__vminu2(c0 | taken[0] | m0, c1 | taken[1] | m1),
+                                 __vminu2(c2 | taken[2] | m2, c3 | taken[3] | m3));
+    // (a piece that is not available has no bit anywhere: its count is 0)
+    const uint32_t hi = __vmaxu2(__vmaxu2(c0 & ~m0, c1 & ~m1), __vmaxu2(c2 & ~m2, c3 & ~m3));
+    uint32_t pmin, pmax;
+    if (G == 32) {
+        pmin = __reduce_min_sync(kFull, min(lo & 0xFFFFu, lo >> 16));
+        pmax = __reduce_max_sync(kFull, max(hi & 0xFFFFu, hi >> 16));
+    } else {
+        // both at once: the minimum, and the maximum as the minimum of its complement
+        uint32_t both = min(lo & 0xFFFFu, lo >> 16) | ((0xFFFFu - max(hi & 0xFFFFu, hi >> 16)) << 16);
+        for (int o = G / 2; o; o >>= 1) both = __vminu2(both, __shfl_xor_sync(gmask, both, o));
+        pmin = both & 0xFFFFu;
+        pmax = 0xFFFFu - (both >> 16);
     }
-    if (__any_sync(kFull, bad)) {
-        r.valid = false;
-        return r;
+    r.valid &= pmin != 0;
+    if (pmin != 0xFFFFu) r.mn = min(r.mn, pmin);
+    r.mx = max(r.mx, pmax);
+    // what this position and the neighbours leave of S[p], from the lane that holds p
+    const uint32_t mine = (k & 1u) ? ((k & 4u) ? t.left[3] : t.left[2]) : ((k & 4u) ? t.left[1] : t.left[0]);
+    const uint32_t sum_n = (__shfl_sync(gmask, mine, wc, G) >> (8 * (k & 2u))) & 0xFFFFu;
+    // every other free position keeps its info without piece p (apply_simple_mask); the bits of
+    // the pieces are the same bits again
+    r.total = 2 * (t.sum_a - sum_n + kept);
+    // the smallest and the largest of them: the first of the lists that is not this position or a
+    // neighbour (lanes 0..5 look at an entry each)
+    const uint32_t el = lane < 6 ? sm.lo[p][lane] : ~0u, eh = lane < 6 ? sm.hi[p][lane] : 0u;
+    auto other = [&](uint32_t e) {
+        const uint32_t j = e & 0xFFFFu;
+        return j != i && j != t.j[0] && j != t.j[1] && j != t.j[2] && j != t.j[3];
+    };
+    const uint32_t bl = (__ballot_sync(gmask, el != ~0u && other(el)) >> gshift) & 63u;
+    const uint32_t bh = (__ballot_sync(gmask, eh != 0u && other(eh)) >> gshift) & 63u;
+    const uint32_t vl = __shfl_sync(gmask, el, bl ? __ffs(bl) - 1 : 0, G) >> 16;
+    const uint32_t vh = __shfl_sync(gmask, eh, bh ? __ffs(bh) - 1 : 0, G) >> 16;
+    if (bl) {
+        r.valid &= vl != 0;
+        r.mn = min(r.mn, vl);
     }
-    r.total += warp_sum(psum);
-    r.mn = min(r.mn, warp_min(pmin));
-    r.mx = max(r.mx, warp_max(pmax));
+    if (bh) r.mx = max(r.mx, vh - 1u);
     return r;
 }
 
@@ -327,14 +379,19 @@ __device__ void load_level(GmSmem& sm, const GmLaunch& P, uint32_t level, uint32
 {
     const uint32_t S = P.n, nb = S - level;
     const uint32_t* src = P.infos + static_cast<size_t>(tri_base(S, level)) * 32;
-    for (uint32_t k = tid; k < nb * 32; k += kThreads) sm.X[k >> 5][k & 31] = src[k];
+    // from L2: in grid mode other blocks wrote most of it
+    for (uint32_t k = 4 * tid; k < nb * 32; k += 4 * kThreads)
+        *reinterpret_cast<uint4*>(&sm.X[k >> 5][k & 31]) = __ldcg(reinterpret_cast<const uint4*>(src + k));
 }
 
-__device__ void store_level(const GmSmem& sm, const GmLaunch& P, uint32_t level, uint32_t tid)
+// rows first, first + stride, ... of the level
+__device__ void store_level(const GmSmem& sm, const GmLaunch& P, uint32_t level, uint32_t tid, uint32_t first,
+                            uint32_t stride)
 {
     const uint32_t S = P.n, nb = S - level;
     uint32_t* dst = P.infos + static_cast<size_t>(tri_base(S, level)) * 32;
-    for (uint32_t k = tid; k < nb * 32; k += kThreads) dst[k] = sm.X[k >> 5][k & 31];
+    for (uint32_t j = first + stride * (tid >> 5); j < nb; j += stride * (kThreads / 32))
+        dst[j * 32 + (tid & 31)] = sm.X[j][tid & 31];
 }
 
 // CUDA_glutton_max_stack::pop (thread 0); returns the restored info index.
@@ -378,6 +435,7 @@ __device__ void push_state(GmSmem& sm, GmState* st, uint32_t S, uint32_t info, u
         }
         st->pushes++;
     }
+    ++sm.pushes;
     const uint32_t last = S - nl;
     const uint32_t last_pos = sm.position_index[last];
     sm.position_index[info] = info;
@@ -420,24 +478,113 @@ __device__ bool grid_sync(GmGrid* g, uint32_t nblocks)
     return ok_s != 0;
 }
 
+// The pass's candidates from rank r0 to r1, tried by one group of G lanes; returns the group's
+// best valid one and marks the invalid ones.
+template <bool GRID, int G>
+__device__ __forceinline__ void try_candidates(GmSmem& sm, GmGrid* g, uint32_t buf, uint32_t nb, uint32_t width,
+                                               uint32_t height, uint32_t r0, uint32_t r1, bool last_level,
+                                               unsigned long long& best_key, uint32_t& best_order)
+{
+    const uint32_t lane = threadIdx.x & (G - 1), gshift = threadIdx.x & 31u & ~(G - 1u);
+    const uint32_t gmask = G == 32 ? kFull : ((1u << (G & 31)) - 1u) << gshift;
+    uint32_t taken[4];
+    {
+        const uint32_t av = sm.avail[lane >> 2] >> (8 * (lane & 3u));  // availability of the lane's pieces
+        auto gone = [&](uint32_t a, uint32_t c) {
+            return ((av >> a) & 1u ? 0u : 0xFFFFu) | ((av >> c) & 1u ? 0u : 0xFFFF0000u);
+        };
+        taken[0] = gone(0, 2);
+        taken[1] = gone(4, 6);
+        taken[2] = gone(1, 3);
+        taken[3] = gone(5, 7);
+    }
+    // the info that holds candidate r0
+    uint32_t i = 0;
+    for (uint32_t step = 128; step; step >>= 1)
+        if (i + step < nb && sm.cum[i + step] <= r0) i += step;
+    // its word and bit
+    uint32_t word = sm.X[i][lane];
+    uint32_t skip = r0 - sm.cum[i], w = 0;
+    {
+        const uint32_t pc = __popc(word);
+        uint32_t x = pc;
+        for (int o = 1; o < G; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(gmask, x, o, G);
+            if (lane >= static_cast<uint32_t>(o)) x += y;
+        }
+        const uint32_t holds = (__ballot_sync(gmask, x > skip) >> gshift);
+        w = __ffs(holds) - 1;
+        skip -= __shfl_sync(gmask, x - pc, w, G);
+    }
+    uint32_t todo = (__ballot_sync(gmask, word != 0) >> gshift) & (G == 32 ? kFull : (1u << (G & 31)) - 1u);
+    todo &= ~0u << w;
+    uint32_t bits = __shfl_sync(gmask, word, w, G);
+    for (; skip; --skip) bits &= bits - 1;
+    TrialSite site;
+    start_site<G>(sm, nb, i, width, height, lane, site);
+    for (uint32_t r = r0; r < r1; ++r) {
+        if (!bits) {
+            todo &= todo - 1;
+            if (!todo) {
+                ++i;
+                word = sm.X[i][lane];
+                todo = (__ballot_sync(gmask, word != 0) >> gshift) & (G == 32 ? kFull : (1u << (G & 31)) - 1u);
+                start_site<G>(sm, nb, i, width, height, lane, site);
+            }
+            w = __ffs(todo) - 1;
+            bits = __shfl_sync(gmask, word, w, G);
+        }
+        const uint32_t b = __ffs(bits) - 1;
+        bits &= bits - 1;
+        const Trial t = trial<G>(sm, site, taken, i, w, b, lane, gshift, gmask);
+        const uint32_t order = (i << 10) | (w << 5) | b;
+        if (!t.valid) {
+            if (lane == 0) {
+                if (GRID) {
+                    atomicOr(&g->inval[buf][i][w], 1u << b);
+                    g->any_invalid[buf] = 1;
+                } else {
+                    atomicOr(&sm.inval[i][w], 1u << b);
+                    sm.any_invalid = 1;
+                }
+            }
+        } else {
+            const unsigned long long key = (static_cast<unsigned long long>(t.total) << 32) | ((t.mx << 16) + t.mn);
+            if (better_candidate(key, order, best_key, best_order, last_level)) {
+                best_key = key;
+                best_order = order;
+            }
+        }
+    }
+}
+
 // One glutton max search.  GRID = false: one block does everything.  GRID = true:
 // every block of a cooperative launch keeps a copy of the level and makes the same
-// decisions; the candidate trials of each validity pass are shared out over the warps
-// of all blocks through global memory (triple-buffered per pass, one grid barrier per
+// decisions; the candidate trials of each validity pass are shared out over the groups
+// of all blocks, results meet in global memory (triple-buffered per pass, one grid barrier per
 // pass), and block 0 keeps the global search record.
-template <bool GRID>
+template <bool GRID, int G>
 __global__ void __launch_bounds__(kThreads, 1) gm_kernel(GmLaunch P)
 {
     extern __shared__ __align__(16) unsigned char gm_raw[];
     GmSmem& sm = *reinterpret_cast<GmSmem*>(gm_raw);
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t S = P.n;
+    const uint32_t S = P.n, height = P.n / P.width;
     GmState* st = P.state;
     GmGrid* g = P.grid;
     const bool owner = !GRID || blockIdx.x == 0;
-    const uint32_t nblocks = gridDim.x;
+    const uint32_t nblocks = GRID ? gridDim.x : 1u, block = GRID ? blockIdx.x : 0u;
     uint32_t pass_no = 0;  // grid mode: passes so far (selects the exchange buffer)
     bool grid_failed = false;
+    // grid mode: rows of a level were stored since the last barrier (every block's share)
+    bool stored = false;
+    auto load_popped = [&](uint32_t at) {
+        if (GRID && stored) {
+            if (!grid_sync(g, nblocks)) grid_failed = true;
+            stored = false;
+        }
+        if (!grid_failed) load_level(sm, P, at, tid);
+    };
     for (uint32_t k = tid; k < 256 * 4; k += kThreads) sm.pieces[k >> 2][k & 3] = P.pieces[k];
     for (uint32_t k = tid; k < P.ncolours * 4 * 32; k += kThreads) (&sm.cc[0][0][0])[k] = P.cc[k];
     for (uint32_t k = tid; k < 256; k += kThreads) {
@@ -451,6 +598,8 @@ __global__ void __launch_bounds__(kThreads, 1) gm_kernel(GmLaunch P)
         sm.new_level = st->new_level;
         sm.pop_index = st->pop_index;
         sm.stop = 0;
+        sm.trials = st->trials;
+        sm.pushes = st->pushes;
     }
     __syncthreads();
     load_level(sm, P, sm.level, tid);
@@ -460,20 +609,13 @@ __global__ void __launch_bounds__(kThreads, 1) gm_kernel(GmLaunch P)
     for (;;) {
         const uint32_t level = sm.level;
         if (level >= S) break;  // full board (level == S) or exhausted (wrapped below 0)
-        if (owner && tid == 0) {
-            const bool stop = (P.push_budget && st->pushes >= P.push_budget) ||
-                              (P.placement_budget && st->trials + st->pushes >= P.placement_budget) ||
-                              (deadline && global_ns() > deadline);
-            sm.stop = stop;
-            if (GRID) g->stop = stop;
-        }
-        if (GRID) {
-            // every block follows block 0's decision
-            if (!grid_sync(g, nblocks)) {
-                grid_failed = true;
-                break;
-            }
-            if (tid == 0) sm.stop = *(volatile uint32_t*)&g->stop;
+        // the budgets are counted alike by every block; the clock is block 0's, left in sm.stop by
+        // the passes of the level before
+        if (tid == 0) {
+            if ((P.push_budget && sm.pushes >= P.push_budget) ||
+                (P.placement_budget && sm.trials + sm.pushes >= P.placement_budget))
+                sm.stop = 1;
+            if (!GRID && deadline && global_ns() > deadline) sm.stop = 1;
         }
         __syncthreads();
         if (sm.stop) break;
@@ -489,7 +631,8 @@ __global__ void __launch_bounds__(kThreads, 1) gm_kernel(GmLaunch P)
                     sm.new_level = 0;
                 }
                 __syncthreads();
-                if (sm.level < S) load_level(sm, P, sm.level, tid);
+                if (sm.level < S) load_popped(sm.level);
+                if (grid_failed) break;
                 __syncthreads();
                 continue;
             }
@@ -498,7 +641,7 @@ __global__ void __launch_bounds__(kThreads, 1) gm_kernel(GmLaunch P)
         // ---- validity fixpoint and scores ----
         bool failed = false;
         for (;;) {
-            level_statistics(sm, nb, tid);
+            level_statistics(sm, S, nb, tid);
             if (sm.any_empty) {
                 failed = true;
                 break;
@@ -509,56 +652,30 @@ __global__ void __launch_bounds__(kThreads, 1) gm_kernel(GmLaunch P)
             }
             if (tid == 0) {
                 sm.any_invalid = 0;
-                sm.next_info = 0;
-                if (owner) st->passes++;
+                sm.trials += sm.sumA;  // every candidate is tried
+                if (owner) {
+                    st->passes++;
+                    if (GRID) g->stop[buf] = deadline && global_ns() > deadline;
+                }
             }
             __syncthreads();
             unsigned long long best_key = 0;
-            uint32_t best_order = ~0u, trials = 0;
+            uint32_t best_order = ~0u;
             const bool last_level = level == S - 1;
-            for (;;) {
-                // work unit: one word (8 pieces x 4 orientations) of one free position's info
-                uint32_t u = 0;
-                if (lane == 0) u = GRID ? atomicAdd(&g->next_info[buf], 1u) : atomicAdd(&sm.next_info, 1u);
-                u = __shfl_sync(kFull, u, 0);
-                const uint32_t i = u >> 5;
-                if (i >= nb) break;
-                for (uint32_t w = u & 31u; w == (u & 31u); ++w) {
-                    uint32_t word = sm.X[i][w];
-                    while (word) {
-                        const uint32_t b = __ffs(word) - 1;
-                        word &= word - 1;
-                        ++trials;
-                        const Trial t = trial(sm, nb, i, w, b, P.width, lane);
-                        const uint32_t order = (i << 10) | (w << 5) | b;
-                        if (!t.valid) {
-                            if (lane == 0) {
-                                if (GRID) {
-                                    atomicOr(&g->inval[buf][i][w], 1u << b);
-                                    g->any_invalid[buf] = 1;
-                                } else {
-                                    atomicOr(&sm.inval[i][w], 1u << b);
-                                    sm.any_invalid = 1;
-                                }
-                            }
-                            continue;
-                        }
-                        const unsigned long long key =
-                            (static_cast<unsigned long long>(t.total) << 32) | ((t.mx << 16) + t.mn);
-                        const bool better = best_order == ~0u ||
-                                            (last_level ? order > best_order
-                                                        : (key > best_key || (key == best_key && order < best_order)));
-                        if (better) {
-                            best_key = key;
-                            best_order = order;
-                        }
-                    }
-                }
+            {
+                const uint32_t groups = nblocks * (kThreads / G);
+                // neighbouring ranges go to different blocks
+                const uint32_t me = (tid / G) * nblocks + block;
+                const uint32_t r0 = static_cast<uint32_t>(static_cast<uint64_t>(sm.sumA) * me / groups);
+                const uint32_t r1 = static_cast<uint32_t>(static_cast<uint64_t>(sm.sumA) * (me + 1) / groups);
+                if (r0 < r1)
+                    try_candidates<GRID, G>(sm, g, buf, nb, P.width, height, r0, r1, last_level, best_key, best_order);
             }
+            __syncwarp();
+            if (G < 32) warp_best(best_key, best_order, last_level);
             if (lane == 0) {
                 sm.warp_key[warp] = best_key;
                 sm.warp_order[warp] = best_order;
-                sm.warp_trials[warp] = trials;
             }
             __syncthreads();
             // this block's best, reduced by warp 0 (a strict total order: any reduction
@@ -567,15 +684,11 @@ __global__ void __launch_bounds__(kThreads, 1) gm_kernel(GmLaunch P)
                 unsigned long long k0 = sm.warp_key[lane];
                 uint32_t o0 = sm.warp_order[lane];
                 warp_best(k0, o0, last_level);
-                unsigned long long tr = sm.warp_trials[lane];
-                for (int d = 16; d; d >>= 1) tr += __shfl_xor_sync(kFull, tr, d);
                 if (lane == 0) {
                     if (GRID) {
-                        atomicAdd(&st->trials, tr);
                         g->blk_key[buf][blockIdx.x] = k0;
                         g->blk_order[buf][blockIdx.x] = o0;
                     } else {
-                        st->trials += tr;
                         sm.best_order = o0;
                     }
                 }
@@ -585,15 +698,12 @@ __global__ void __launch_bounds__(kThreads, 1) gm_kernel(GmLaunch P)
                     grid_failed = true;
                     break;
                 }
-                // the buffer of the pass before last is free again: block 0 clears it
-                if (blockIdx.x == 0) {
-                    const uint32_t old = (pass_no + 2) % 3;
-                    for (uint32_t k = tid; k < S * 32; k += kThreads) (&g->inval[old][0][0])[k] = 0;
-                    if (tid == 0) {
-                        g->any_invalid[old] = 0;
-                        g->next_info[old] = 0;
-                    }
-                }
+                stored = false;
+                // the buffer of the pass before last is free again: every block clears its rows
+                const uint32_t old = (pass_no + 2) % 3;
+                for (uint32_t j = block + nblocks * warp; j < S; j += nblocks * (kThreads / 32))
+                    g->inval[old][j][lane] = 0;
+                if (block == 0 && tid == 0) g->any_invalid[old] = 0;
                 if (warp == 0) {
                     // the blocks' bests, 32 at a time (the loads overlap instead of
                     // waiting on L2 one block after another)
@@ -611,6 +721,7 @@ __global__ void __launch_bounds__(kThreads, 1) gm_kernel(GmLaunch P)
                     if (lane == 0) {
                         sm.any_invalid = *(volatile uint32_t*)&g->any_invalid[buf];
                         sm.best_order = o0;
+                        sm.stop = *(volatile uint32_t*)&g->stop[buf];
                     }
                 }
                 ++pass_no;
@@ -618,8 +729,11 @@ __global__ void __launch_bounds__(kThreads, 1) gm_kernel(GmLaunch P)
             __syncthreads();
             if (!sm.any_invalid) break;
             if (GRID) {
-                for (uint32_t k = tid; k < nb * 32; k += kThreads)
-                    sm.X[k >> 5][k & 31] &= ~(*(volatile uint32_t*)&g->inval[buf][k >> 5][k & 31]);
+                for (uint32_t k = 4 * tid; k < nb * 32; k += 4 * kThreads) {
+                    const uint4 v = __ldcg(reinterpret_cast<const uint4*>(&g->inval[buf][k >> 5][k & 31]));
+                    uint4& x = *reinterpret_cast<uint4*>(&sm.X[k >> 5][k & 31]);
+                    x = make_uint4(x.x & ~v.x, x.y & ~v.y, x.z & ~v.z, x.w & ~v.w);
+                }
             } else {
                 for (uint32_t k = tid; k < nb * 32; k += kThreads) sm.X[k >> 5][k & 31] &= ~sm.inval[k >> 5][k & 31];
             }
@@ -635,7 +749,8 @@ __global__ void __launch_bounds__(kThreads, 1) gm_kernel(GmLaunch P)
                 sm.new_level = 0;
             }
             __syncthreads();
-            if (sm.level < S) load_level(sm, P, sm.level, tid);
+            if (sm.level < S) load_popped(sm.level);
+            if (grid_failed) break;
             __syncthreads();
             continue;
         }
@@ -645,10 +760,10 @@ __global__ void __launch_bounds__(kThreads, 1) gm_kernel(GmLaunch P)
         const uint32_t pos = sm.position_index[bi];
         if (tid == 0) sm.X[bi][bw] &= ~(1u << bb);
         __syncthreads();
-        // the level keeps its remaining candidates for a later pop (in grid mode every
-        // block writes the same values and reads back only its own writes)
-        store_level(sm, P, level, tid);
-        __threadfence_block();
+        // the level keeps its remaining candidates for a later pop.  In grid mode each block
+        // writes its share, and a pop reads the level after a barrier.
+        store_level(sm, P, level, tid, block, nblocks);
+        stored = true;
         const uint32_t pm_word = ~(0xFu << (4 * (bb / 4)));
         // the next level moves the last info into the chosen slot; an empty
         // result there stops the reference's apply before its push
@@ -696,7 +811,8 @@ __global__ void __launch_bounds__(kThreads, 1) gm_kernel(GmLaunch P)
             __syncthreads();
             if (tid == 0) pop_state(sm, st, S, owner);
             __syncthreads();
-            load_level(sm, P, sm.level, tid);
+            load_popped(sm.level);
+            if (grid_failed) break;
         }
         if (tid == 0) sm.new_level = 1;
         __syncthreads();
@@ -709,9 +825,10 @@ __global__ void __launch_bounds__(kThreads, 1) gm_kernel(GmLaunch P)
         st->level = level;
         st->new_level = sm.new_level;
         st->pop_index = sm.pop_index;
+        st->trials = sm.trials;
         st->status = grid_failed ? 3 : (level == S ? 0 : (level > S ? 2 : 1));
     }
-    if (sm.level < S) store_level(sm, P, sm.level, tid);
+    if (sm.level < S) store_level(sm, P, sm.level, tid, 0, 1);
     for (uint32_t k = tid; k < 256; k += kThreads) {
         st->position_index[k] = sm.position_index[k];
         st->info_index[k] = sm.info_index[k];
@@ -723,24 +840,38 @@ __global__ void __launch_bounds__(kThreads, 1) gm_kernel(GmLaunch P)
 
 size_t gm_smem_bytes() { return sizeof(GmSmem); }
 
+namespace {
+
+// lanes of a trial's group: the words that hold pieces
+template <bool GRID>
+const void* gm_symbol(uint32_t n)
+{
+    if (n <= 64) return reinterpret_cast<const void*>(&gm_kernel<GRID, 8>);
+    if (n <= 128) return reinterpret_cast<const void*>(&gm_kernel<GRID, 16>);
+    return reinterpret_cast<const void*>(&gm_kernel<GRID, 32>);
+}
+
+}  // namespace
+
 cudaError_t launch_gm(const GmLaunch& P, cudaStream_t stream)
 {
     const size_t smem = sizeof(GmSmem);
-    cudaError_t e = cudaFuncSetAttribute(gm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem));
+    const void* fn = gm_symbol<false>(P.n);
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
-    gm_kernel<false><<<1, kThreads, smem, stream>>>(P);
-    return cudaGetLastError();
+    GmLaunch copy = P;
+    void* args[] = {&copy};
+    return cudaLaunchKernel(fn, dim3(1), dim3(kThreads), args, smem, stream);
 }
 
 cudaError_t launch_gm_grid(const GmLaunch& P, uint32_t blocks, cudaStream_t stream)
 {
     const size_t smem = sizeof(GmSmem);
-    cudaError_t e = cudaFuncSetAttribute(gm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem));
+    const void* fn = gm_symbol<true>(P.n);
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
     int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gm_kernel<true>, kThreads, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kThreads, smem);
     if (e != cudaSuccess) return e;
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
@@ -749,8 +880,7 @@ cudaError_t launch_gm_grid(const GmLaunch& P, uint32_t blocks, cudaStream_t stre
         return cudaErrorCooperativeLaunchTooLarge;
     GmLaunch copy = P;
     void* args[] = {&copy};
-    return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(&gm_kernel<true>), dim3(blocks), dim3(kThreads),
-                                       args, smem, stream);
+    return cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(kThreads), args, smem, stream);
 }
 
 }  // namespace emp

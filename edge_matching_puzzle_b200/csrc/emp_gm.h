@@ -33,9 +33,9 @@ constexpr uint32_t kMaxGridBlocks = 256;
 struct GmGrid {
     uint32_t bar_count, bar_gen;  // grid barrier
     int error;                    // a barrier wait ran out of time
-    uint32_t stop;                // block 0's decision at the top of a level
-    uint32_t any_invalid[3];      // per pass buffer (pass number mod 3)
-    uint32_t next_info[3];
+    uint32_t stop[3];             // per pass buffer (pass number mod 3): block 0's clock ran out
+    uint32_t any_invalid[3];
+    uint32_t pad[3];              // the rows below are read 16 bytes at a time
     uint32_t inval[3][256][32];
     unsigned long long blk_key[3][kMaxGridBlocks];
     uint32_t blk_order[3][kMaxGridBlocks];
