@@ -60,14 +60,6 @@ __device__ __forceinline__ uint64_t ldg64(const uint32_t* p)
     return __ldg(reinterpret_cast<const unsigned long long*>(p));
 }
 
-// bits of `v` at and above bit `s` (0..64)
-__device__ __forceinline__ uint64_t from_bit(uint64_t v, uint32_t s)
-{
-    uint64_t ones;
-    asm("shl.b64 %0, %1, %2;" : "=l"(ones) : "l"(~0ull), "r"(s));  // a shift by 64 gives 0
-    return v & ones;
-}
-
 template <int NW>
 struct Search {
     uint64_t orig, nodes, sols, steps;

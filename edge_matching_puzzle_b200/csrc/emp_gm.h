@@ -31,11 +31,10 @@ struct GmState {
 // Exchange area of the multi-block search (one per search, global memory).
 constexpr uint32_t kMaxGridBlocks = 256;
 struct GmGrid {
-    uint32_t bar_count, bar_gen;  // grid barrier
     int error;                    // a barrier wait ran out of time
-    uint32_t stop[3];             // per pass buffer (pass number mod 3): block 0's clock ran out
-    uint32_t any_invalid[3];
-    uint32_t pad[3];              // the rows below are read 16 bytes at a time
+    uint32_t arrive[3];           // per pass buffer (pass number mod 3): arrivals and flags
+    uint32_t extra[3];            // barriers outside the passes
+    uint32_t pad[5];              // the rows below are read 16 bytes at a time
     uint32_t inval[3][256][32];
     unsigned long long blk_key[3][kMaxGridBlocks];
     uint32_t blk_order[3][kMaxGridBlocks];
