@@ -112,7 +112,11 @@ emp_status expand(emp_bt_plan_t& pl)
     DeviceBuffer parents, parent_puzzle, children, child_puzzle, counts, offsets, bsums, grand, lv;
     CUDA_TRY(lv.alloc(sizeof(unsigned long long) * 2 * P));
     CUDA_TRY(cudaMemsetAsync(lv.p, 0, lv.bytes, st));
-    CUDA_TRY(parent_puzzle.alloc(sizeof(uint32_t) * P));
+    // a plain expansion takes its first levels in one launch while they have at most kFew prefixes
+    // (a dump keeps every level, and per-puzzle depths are decided here level by level)
+    constexpr uint32_t kFew = 4096;
+    const bool few = !pl.dump && !pl.adaptive && P <= kFew;
+    CUDA_TRY(parent_puzzle.alloc(sizeof(uint32_t) * (few ? kFew : P)));
     {
         // subtrees are queued puzzle by puzzle, smaller puzzles first: under a
         // deadline the cheap instances of a mixed batch finish before the threads
@@ -125,29 +129,54 @@ emp_status expand(emp_bt_plan_t& pl)
         CUDA_TRY(cudaMemcpyAsync(parent_puzzle.p, ids.data(), sizeof(uint32_t) * P, cudaMemcpyHostToDevice, st));
         CUDA_TRY(cudaStreamSynchronize(st));
     }
-    CUDA_TRY(parents.alloc(2));
-    CUDA_TRY(grand.alloc(sizeof(uint64_t)));
+    CUDA_TRY(parents.alloc(few ? sizeof(uint16_t) * kFew * pl.depth : 2));
     uint64_t np = P;
     unsigned long long* lnodes = lv.as<unsigned long long>();
     // per puzzle split depths: a puzzle stops expanding (is frozen) once it has
-    // split_subtrees prefixes, reaches its depth limit or runs out of prefixes
-    DeviceBuffer frozen_dev;
-    std::vector<uint8_t> frozen(P, 0);
-    std::vector<uint32_t> cap(P);
-    std::vector<unsigned long long> seen(P, 0), now(P, 0);
+    // split_subtrees prefixes, reaches its depth limit or runs out of prefixes.  The device keeps
+    // the flags, so that a level waits for the host once.
+    DeviceBuffer frozen_dev, frozen_next, seen, limit;
     uint32_t levels = pl.depth;
     pl.puzzle_depth.assign(P, pl.depth);
+    CUDA_TRY(grand.alloc(2 * sizeof(uint64_t)));  // prefixes of the level, puzzles not frozen
     if (pl.adaptive) {
-        CUDA_TRY(frozen_dev.alloc(P));
-        CUDA_TRY(cudaMemsetAsync(frozen_dev.p, 0, P, st));
+        std::vector<uint32_t> cap(P);
         levels = 0;
         for (uint32_t i = 0; i < P; ++i) {
             const uint32_t lim = pl.cfg.split_depth ? std::min<uint32_t>(pl.cfg.split_depth, 64u) : 64u;
             cap[i] = std::max<uint32_t>(1u, std::min<uint32_t>(lim, pl.puzzles[i]->model.n - 1));
             levels = std::max(levels, cap[i]);
         }
+        CUDA_TRY(frozen_dev.alloc(P));
+        CUDA_TRY(frozen_next.alloc(P));
+        CUDA_TRY(seen.alloc(sizeof(unsigned long long) * P));
+        CUDA_TRY(limit.alloc(sizeof(uint32_t) * P));
+        CUDA_TRY(pl.puzzle_depth_dev.alloc(sizeof(uint32_t) * P));
+        CUDA_TRY(cudaMemsetAsync(frozen_dev.p, 0, P, st));
+        CUDA_TRY(cudaMemsetAsync(seen.p, 0, seen.bytes, st));
+        CUDA_TRY(cudaMemcpyAsync(limit.p, cap.data(), sizeof(uint32_t) * P, cudaMemcpyHostToDevice, st));
+        CUDA_TRY(cudaStreamSynchronize(st));
     }
     uint32_t level = 0;
+    if (few) {
+        DeviceBuffer done;
+        uint32_t got[3] = {0, 0, 0};
+        CUDA_TRY(children.alloc(sizeof(uint16_t) * kFew * pl.depth));
+        CUDA_TRY(child_puzzle.alloc(sizeof(uint32_t) * kFew));
+        CUDA_TRY(done.alloc(sizeof(got)));
+        CUDA_TRY(emp::launch_expand_few(L, parents.as<uint16_t>(), children.as<uint16_t>(), parent_puzzle.as<uint32_t>(),
+                                        child_puzzle.as<uint32_t>(), P, levels, kFew, lnodes, lnodes + P,
+                                        done.as<uint32_t>(), st));
+        CUDA_TRY(cudaMemcpyAsync(got, done.p, sizeof(got), cudaMemcpyDeviceToHost, st));
+        CUDA_TRY(cudaStreamSynchronize(st));
+        np = got[0];
+        level = got[1];
+        if (got[2]) {
+            std::swap(parents, children);
+            std::swap(parent_puzzle, child_puzzle);
+        }
+        if (!np) levels = level;  // the search ends above the split depth
+    }
     for (; level < levels; ++level) {
         CUDA_TRY(counts.reserve(sizeof(uint32_t) * std::max<uint64_t>(np, 1)));
         CUDA_TRY(offsets.reserve(sizeof(uint64_t) * std::max<uint64_t>(np, 1)));
@@ -158,9 +187,17 @@ emp_status expand(emp_bt_plan_t& pl)
                                            fz, st));
         CUDA_TRY(emp::launch_scan(counts.as<uint32_t>(), np, offsets.as<uint64_t>(), bsums.as<uint64_t>(),
                                   grand.as<uint64_t>(), st));
-        uint64_t total = 0;
-        CUDA_TRY(cudaMemcpyAsync(&total, grand.p, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
+        uint64_t got[2] = {0, 0};
+        if (pl.adaptive) {
+            CUDA_TRY(cudaMemsetAsync(grand.as<uint64_t>() + 1, 0, sizeof(uint64_t), st));
+            CUDA_TRY(emp::launch_freeze(lnodes, seen.as<unsigned long long>(), limit.as<uint32_t>(), P, level,
+                                        pl.cfg.split_subtrees, frozen_dev.as<uint8_t>(), frozen_next.as<uint8_t>(),
+                                        pl.puzzle_depth_dev.as<uint32_t>(),
+                                        grand.as<unsigned long long>() + 1, st));
+        }
+        CUDA_TRY(cudaMemcpyAsync(got, grand.p, (pl.adaptive ? 2 : 1) * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
         CUDA_TRY(cudaStreamSynchronize(st));
+        const uint64_t total = got[0];
         CUDA_TRY(children.reserve(sizeof(uint16_t) * std::max<uint64_t>(total, 1) * (level + 1)));
         CUDA_TRY(child_puzzle.reserve(sizeof(uint32_t) * std::max<uint64_t>(total, 1)));
         CUDA_TRY(emp::launch_expand_frozen(L, parents.as<uint16_t>(), parent_puzzle.as<uint32_t>(), np, level,
@@ -184,21 +221,8 @@ emp_status expand(emp_bt_plan_t& pl)
         }
         np = total;
         if (pl.adaptive) {
-            // placements of this level per puzzle = its prefixes after this level
-            CUDA_TRY(cudaMemcpyAsync(now.data(), lnodes, sizeof(unsigned long long) * P, cudaMemcpyDeviceToHost, st));
-            CUDA_TRY(cudaStreamSynchronize(st));
-            bool all = true;
-            for (uint32_t i = 0; i < P; ++i) {
-                if (frozen[i]) continue;
-                const unsigned long long prefixes = now[i] - seen[i];
-                seen[i] = now[i];
-                pl.puzzle_depth[i] = level + 1;
-                if (prefixes >= pl.cfg.split_subtrees || level + 1 >= cap[i] || !prefixes) frozen[i] = 1;
-                all = all && frozen[i];
-            }
-            CUDA_TRY(cudaMemcpyAsync(frozen_dev.p, frozen.data(), P, cudaMemcpyHostToDevice, st));
-            CUDA_TRY(cudaStreamSynchronize(st));
-            if (all) {
+            std::swap(frozen_dev, frozen_next);
+            if (!got[1]) {
                 ++level;
                 break;
             }
@@ -216,9 +240,8 @@ emp_status expand(emp_bt_plan_t& pl)
     CUDA_TRY(cudaStreamSynchronize(st));
     pl.n_all = np;
     if (pl.adaptive) {
-        CUDA_TRY(pl.puzzle_depth_dev.alloc(sizeof(uint32_t) * P));
-        CUDA_TRY(cudaMemcpyAsync(pl.puzzle_depth_dev.p, pl.puzzle_depth.data(), sizeof(uint32_t) * P,
-                                 cudaMemcpyHostToDevice, st));
+        CUDA_TRY(cudaMemcpyAsync(pl.puzzle_depth.data(), pl.puzzle_depth_dev.p, sizeof(uint32_t) * P,
+                                 cudaMemcpyDeviceToHost, st));
         CUDA_TRY(cudaStreamSynchronize(st));
     }
     pl.prefixes = std::move(parents);

@@ -46,7 +46,69 @@ __device__ __forceinline__ uint64_t global_ns()
 }
 
 // ---------------------------------------------------------------------------
-// Prefix expansion.  mode 0: count children; mode 1: write children.
+// Prefix expansion.
+
+// The children of one prefix in the reference's order: counts them, or (EMIT) writes each with
+// the prefix before it, from child number `out` on.
+template <bool EMIT>
+__device__ __forceinline__ uint32_t expand_parent(const BtLaunch& P, const uint16_t* __restrict__ pre, uint32_t pz,
+                                                  uint32_t level, uint64_t out, uint16_t* __restrict__ children,
+                                                  uint32_t* __restrict__ child_puzzle, bool* last)
+{
+    const uint32_t* tb = P.tables + P.puzzle_offset[pz];
+    const uint32_t n = ldg(tb + H_N), ncol = ldg(tb + H_NCOL), desc_off = ldg(tb + H_DESC);
+    uint64_t av[kMaxAvailWords];
+    uint32_t stk[kMaxExpandDepth];
+    const uint32_t aw = ldg(tb + H_AWORDS), init = ldg(tb + H_INIT);
+    for (uint32_t w = 0; w < aw; ++w) av[w] = ldg64(tb + init + 2 * w);
+    for (uint32_t l = 0; l < level; ++l) {
+        const LevelDesc d = load_desc(tb, desc_off, l);
+        const uint32_t t = pre[l];
+        av[d.aoff() + (t >> 6)] &= ~(0xFull << (t & 60u));
+        stk[l] = ldg(tb + d.d5 + t) & 0xFFFFFu;
+    }
+    uint32_t cnt = 0;
+    *last = level == n - 1;
+    if (level < n) {
+        const LevelDesc d = load_desc(tb, desc_off, level);
+        const uint32_t kw = d.kw();
+        const uint32_t row = d.row(stk[d.level_a()], stk[d.level_b()]);
+        uint64_t R[kMaxKindWords];
+        for (uint32_t w = 0; w < kw; ++w) R[w] = ldg64(tb + row + 2 * w) & av[d.aoff() + w];
+        for (uint32_t j = 0; j < d.nextra(); ++j) {
+            const uint32_t sd = d.extra_side(j);
+            const uint32_t c = facing_colour(stk[d.extra_level(j)], sd);
+            const uint32_t* sm = tb + d.d4 + ((sd * ncol + c) * kw) * 2;
+            for (uint32_t w = 0; w < kw; ++w) R[w] &= ldg64(sm + 2 * w);
+        }
+        for (uint32_t w = 0; w < kw; ++w) {
+            while (R[w]) {
+                const uint32_t t = w * 64 + __ffsll(R[w]) - 1;
+                if (EMIT) {
+                    uint16_t* c = children + out * (level + 1);
+                    for (uint32_t l = 0; l < level; ++l) c[l] = pre[l];
+                    c[level] = static_cast<uint16_t>(t);
+                    if (child_puzzle) child_puzzle[out] = pz;
+                    ++out;
+                }
+                ++cnt;
+                if (level == 0) {  // position 0 keeps its first transition (emp_strategy.h:389)
+                    w = kw;
+                    break;
+                }
+                if ((ldg(tb + d.d5 + t) >> 20) & 1u) {
+                    const uint32_t* ex = tb + d.d6 + t * kw * 2;
+                    for (uint32_t ww = 0; ww < kw; ++ww) R[ww] &= ldg64(ex + 2 * ww);
+                } else {
+                    R[w] &= ~(1ull << (t & 63));
+                }
+            }
+        }
+    }
+    return cnt;
+}
+
+// One level.  mode 0: count children; mode 1: write children.
 __global__ void expand_kernel(BtLaunch P, const uint16_t* __restrict__ parents,
                               const uint32_t* __restrict__ parent_puzzle, uint64_t n_parents,
                               uint32_t level, uint32_t* __restrict__ counts,
@@ -71,64 +133,100 @@ __global__ void expand_kernel(BtLaunch P, const uint16_t* __restrict__ parents,
             }
             continue;
         }
-        const uint32_t* tb = P.tables + P.puzzle_offset[pz];
-        const uint32_t n = ldg(tb + H_N), ncol = ldg(tb + H_NCOL), desc_off = ldg(tb + H_DESC);
-        uint64_t av[kMaxAvailWords];
-        uint32_t stk[kMaxExpandDepth];
-        const uint32_t aw = ldg(tb + H_AWORDS), init = ldg(tb + H_INIT);
-        for (uint32_t w = 0; w < aw; ++w) av[w] = ldg64(tb + init + 2 * w);
-        const uint16_t* pre = parents + i * level;
-        for (uint32_t l = 0; l < level; ++l) {
-            const LevelDesc d = load_desc(tb, desc_off, l);
-            const uint32_t t = pre[l];
-            av[d.aoff() + (t >> 6)] &= ~(0xFull << (t & 60u));
-            stk[l] = ldg(tb + d.d5 + t) & 0xFFFFFu;
-        }
-        uint32_t cnt = 0;
-        if (level < n) {
-            const LevelDesc d = load_desc(tb, desc_off, level);
-            const uint32_t kw = d.kw();
-            const uint32_t row = d.row(stk[d.level_a()], stk[d.level_b()]);
-            uint64_t R[kMaxKindWords];
-            for (uint32_t w = 0; w < kw; ++w) R[w] = ldg64(tb + row + 2 * w) & av[d.aoff() + w];
-            for (uint32_t j = 0; j < d.nextra(); ++j) {
-                const uint32_t sd = d.extra_side(j);
-                const uint32_t c = facing_colour(stk[d.extra_level(j)], sd);
-                const uint32_t* sm = tb + d.d4 + ((sd * ncol + c) * kw) * 2;
-                for (uint32_t w = 0; w < kw; ++w) R[w] &= ldg64(sm + 2 * w);
-            }
-            uint64_t out = mode ? offsets[i] : 0;
-            for (uint32_t w = 0; w < kw; ++w) {
-                while (R[w]) {
-                    const uint32_t t = w * 64 + __ffsll(R[w]) - 1;
-                    if (mode) {
-                        uint16_t* c = children + out * (level + 1);
-                        for (uint32_t l = 0; l < level; ++l) c[l] = pre[l];
-                        c[level] = static_cast<uint16_t>(t);
-                        if (child_puzzle) child_puzzle[out] = pz;
-                        ++out;
-                    }
-                    ++cnt;
-                    if (level == 0) {  // position 0 keeps its first transition (emp_strategy.h:389)
-                        w = kw;
-                        break;
-                    }
-                    if ((ldg(tb + d.d5 + t) >> 20) & 1u) {
-                        const uint32_t* ex = tb + d.d6 + t * kw * 2;
-                        for (uint32_t ww = 0; ww < kw; ++ww) R[ww] &= ldg64(ex + 2 * ww);
-                    } else {
-                        R[w] &= ~(1ull << (t & 63));
-                    }
-                }
-            }
-        }
-        if (!mode) {
+        bool last;
+        if (mode) {
+            expand_parent<true>(P, parents + i * level, pz, level, offsets[i], children, child_puzzle, &last);
+        } else {
+            const uint32_t cnt = expand_parent<false>(P, parents + i * level, pz, level, 0, nullptr, nullptr, &last);
             counts[i] = cnt;
+            // one addition for the lanes at work on the same puzzle (6.3 million parents of a 10x10
+            // plan added to one address)
+            const unsigned peers = __match_any_sync(__activemask(), pz);
+            const uint32_t sum = __reduce_add_sync(peers, cnt);
+            if (sum && (threadIdx.x & 31u) == __ffs(peers) - 1) {
+                atomicAdd(&level_nodes[pz], (unsigned long long)sum);
+                if (last) atomicAdd(&level_sols[pz], (unsigned long long)sum);
+            }
+        }
+    }
+}
+
+// Per-puzzle split depths: after a level's count pass, a puzzle that is not frozen yet has `nodes`
+// less `seen` prefixes of length level + 1; it freezes once they are `target` or none, or its
+// depth limit is reached.  next: the flags of the next level; still[0] counts the others.
+__global__ void freeze_kernel(const unsigned long long* __restrict__ nodes, unsigned long long* __restrict__ seen,
+                              const uint32_t* __restrict__ limit, uint32_t n_puzzles, uint32_t level, uint32_t target,
+                              const uint8_t* __restrict__ frozen, uint8_t* __restrict__ next,
+                              uint32_t* __restrict__ depth, unsigned long long* __restrict__ still)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    bool open = false;
+    if (i < n_puzzles) {
+        uint8_t f = frozen[i];
+        if (!f) {
+            const unsigned long long prefixes = nodes[i] - seen[i];
+            seen[i] = nodes[i];
+            depth[i] = level + 1;
+            f = prefixes >= target || level + 1 >= limit[i] || !prefixes;
+            open = !f;
+        }
+        next[i] = f;
+    }
+    const unsigned ballot = __ballot_sync(kFull, open);
+    if ((threadIdx.x & 31u) == 0 && ballot) atomicAdd(still, (unsigned long long)__popc(ballot));
+}
+
+__device__ uint64_t block_exclusive_scan(uint64_t v, uint64_t* sh, uint64_t& total);
+
+// The first levels, while they have few prefixes, in one block and one launch: a level a launch
+// costs five launches and a wait of the host, 60 us, for microseconds of work (an expansion to
+// level 12 took 0.8 ms of a 5x5 count's 1.2 ms).  The prefixes of a level are in the one or the
+// other of two buffers of `capacity` rows of `max_level` transitions; the block stops before
+// `max_level` or the level whose prefixes would not fit.  out: [0] prefixes, [1] their length,
+// [2] the buffer they are in.
+constexpr uint32_t kFewThreads = 1024;
+
+__global__ void __launch_bounds__(kFewThreads) expand_few_kernel(BtLaunch P, uint16_t* buf0, uint16_t* buf1, uint32_t* pz0, uint32_t* pz1,
+                                                                 uint32_t n_roots, uint32_t max_level, uint32_t capacity,
+                                                                 unsigned long long* level_nodes,
+                                                                 unsigned long long* level_sols, uint32_t* out)
+{
+    __shared__ uint64_t sh[32];
+    uint32_t np = n_roots, which = 0, level = 0;
+    for (; level < max_level && np; ++level) {
+        const uint16_t* parents = which ? buf1 : buf0;
+        const uint32_t* puzzle = which ? pz1 : pz0;
+        uint16_t* children = which ? buf0 : buf1;
+        uint32_t* child_puzzle = which ? pz0 : pz1;
+        // consecutive parents to a thread, so that the scan keeps the prefixes in order
+        const uint32_t each = (np + kFewThreads - 1) / kFewThreads;
+        const uint32_t i0 = min(threadIdx.x * each, np), i1 = min(i0 + each, np);
+        uint32_t mine = 0;
+        bool last = false;
+        for (uint32_t i = i0; i < i1; ++i)
+            mine += expand_parent<false>(P, parents + static_cast<uint64_t>(i) * level, puzzle[i], level, 0, nullptr,
+                                         nullptr, &last);
+        uint64_t total;
+        uint64_t at = block_exclusive_scan(mine, sh, total);
+        if (total > capacity) break;
+        for (uint32_t i = i0; i < i1; ++i) {
+            const uint32_t pz = puzzle[i];
+            const uint32_t cnt = expand_parent<true>(P, parents + static_cast<uint64_t>(i) * level, pz, level, at,
+                                                     children, child_puzzle, &last);
+            at += cnt;
             if (cnt) {
                 atomicAdd(&level_nodes[pz], (unsigned long long)cnt);
-                if (level == n - 1) atomicAdd(&level_sols[pz], (unsigned long long)cnt);
+                if (last) atomicAdd(&level_sols[pz], (unsigned long long)cnt);
             }
         }
+        np = static_cast<uint32_t>(total);
+        which ^= 1u;
+        __syncthreads();  // the children are this block's next parents
+    }
+    if (threadIdx.x == 0) {
+        out[0] = np;
+        out[1] = level;
+        out[2] = which;
     }
 }
 
@@ -1363,6 +1461,24 @@ cudaError_t launch_expand_frozen(const BtLaunch& P, const uint16_t* parents, con
     expand_kernel<<<(unsigned)blocks, threads, 0, stream>>>(P, parents, parent_puzzle, n_parents, level, counts,
                                                             offsets, children, child_puzzle, level_nodes,
                                                             level_sols, mode, frozen);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_freeze(const unsigned long long* nodes, unsigned long long* seen, const uint32_t* limit,
+                          uint32_t n_puzzles, uint32_t level, uint32_t target, const uint8_t* frozen, uint8_t* next,
+                          uint32_t* depth, unsigned long long* still, cudaStream_t stream)
+{
+    freeze_kernel<<<(n_puzzles + 255) / 256, 256, 0, stream>>>(nodes, seen, limit, n_puzzles, level, target, frozen, next,
+                                                               depth, still);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_expand_few(const BtLaunch& P, uint16_t* buf0, uint16_t* buf1, uint32_t* pz0, uint32_t* pz1,
+                              uint32_t n_roots, uint32_t max_level, uint32_t capacity, unsigned long long* level_nodes,
+                              unsigned long long* level_sols, uint32_t* out, cudaStream_t stream)
+{
+    expand_few_kernel<<<1, kFewThreads, 0, stream>>>(P, buf0, buf1, pz0, pz1, n_roots, max_level, capacity, level_nodes,
+                                                     level_sols, out);
     return cudaGetLastError();
 }
 

@@ -105,6 +105,14 @@ cudaError_t launch_expand(const BtLaunch& P, const uint16_t* parents, const uint
                           uint64_t n_parents, uint32_t level, uint32_t* counts, const uint64_t* offsets,
                           uint16_t* children, uint32_t* child_puzzle, unsigned long long* level_nodes,
                           unsigned long long* level_sols, int mode, cudaStream_t stream);
+// Which puzzles of a plan with per-puzzle split depths stop after this level (emp_bt.cu, freeze_kernel).
+cudaError_t launch_freeze(const unsigned long long* nodes, unsigned long long* seen, const uint32_t* limit,
+                          uint32_t n_puzzles, uint32_t level, uint32_t target, const uint8_t* frozen, uint8_t* next,
+                          uint32_t* depth, unsigned long long* still, cudaStream_t stream);
+// The first levels of an expansion in one launch (emp_bt.cu, expand_few_kernel).
+cudaError_t launch_expand_few(const BtLaunch& P, uint16_t* buf0, uint16_t* buf1, uint32_t* pz0, uint32_t* pz1,
+                              uint32_t n_roots, uint32_t max_level, uint32_t capacity, unsigned long long* level_nodes,
+                              unsigned long long* level_sols, uint32_t* out, cudaStream_t stream);
 cudaError_t launch_scan(const uint32_t* counts, uint64_t n, uint64_t* offsets, uint64_t* block_sums,
                         uint64_t* grand_total, cudaStream_t stream);
 uint64_t scan_block_sum_words(uint64_t n);
