@@ -37,27 +37,32 @@ struct emp_mlp_t {
 
 namespace {
 
-// training workspace for up to `rows` rows
+// training workspace for up to `rows` rows, one allocation
 struct Work {
-    DeviceBuffer h1, h2, s, ds, dh2, dh1, grad, loss;
+    DeviceBuffer all;
     emp::MlpWork w;
     cudaError_t alloc(uint64_t rows)
     {
-        const uint64_t H = emp::kMlpHidden;
-        cudaError_t e;
-        if ((e = h1.alloc(4 * rows * H)) || (e = h2.alloc(4 * rows * H)) || (e = s.alloc(4 * rows)) ||
-            (e = ds.alloc(4 * rows)) || (e = dh2.alloc(4 * rows * H)) || (e = dh1.alloc(4 * rows * H)) ||
-            (e = grad.alloc(4ull * emp::kMlpParams)) || (e = loss.alloc(2 * sizeof(double))))
-            return e;
+        const uint64_t H = emp::kMlpHidden, R = (rows + 3) / 4 * 4;  // every part on 16 bytes
+        const uint64_t parts = (emp::mlp_part_floats(rows) + 3) / 4 * 4, grad = (emp::kMlpParams + 3) / 4 * 4;
+        const cudaError_t e = all.alloc(4 * (4 * R * H + 2 * R + grad + parts) + 2 * sizeof(double));
+        if (e) return e;
+        float* p = all.as<float>();
+        auto take = [&p](uint64_t n) {
+            float* q = p;
+            p += n;
+            return q;
+        };
         w.rows = rows;
-        w.h1 = h1.as<float>();
-        w.h2 = h2.as<float>();
-        w.s = s.as<float>();
-        w.ds = ds.as<float>();
-        w.dh2 = dh2.as<float>();
-        w.dh1 = dh1.as<float>();
-        w.grad = grad.as<float>();
-        w.loss = loss.as<double>();
+        w.h1 = take(R * H);
+        w.h2 = take(R * H);
+        w.dh2 = take(R * H);
+        w.dh1 = take(R * H);
+        w.s = take(R);
+        w.ds = take(R);
+        w.grad = take(grad);
+        w.parts = take(parts);
+        w.loss = reinterpret_cast<double*>(p);
         return cudaSuccess;
     }
 };
@@ -257,7 +262,7 @@ extern "C" emp_status emp_mlp_score_f32(emp_mlp model, const float* features, ui
     CUDA_TRY(w.alloc(n));
     CUDA_TRY(cudaMemcpy(x.p, features, 4ull * emp::kMlpIn * n, cudaMemcpyHostToDevice));
     CUDA_TRY(emp::mlp_forward_f32(model->dev(), w.w, x.as<float>(), n, nullptr));
-    CUDA_TRY(cudaMemcpy(scores, w.s.p, 4ull * n, cudaMemcpyDeviceToHost));
+    CUDA_TRY(cudaMemcpy(scores, w.w.s, 4ull * n, cudaMemcpyDeviceToHost));
     return EMP_OK;
 }
 
@@ -280,9 +285,9 @@ extern "C" emp_status emp_mlp_loss_grad(emp_mlp model, const float* features, co
     CUDA_TRY(emp::mlp_forward_f32(model->dev(), w.w, x.as<float>(), n, nullptr));
     CUDA_TRY(emp::mlp_loss_backward_f32(model->dev(), w.w, x.as<float>(), y.as<float>(), w8.as<float>(), n, nullptr));
     double l[2];
-    CUDA_TRY(cudaMemcpy(l, w.loss.p, sizeof(l), cudaMemcpyDeviceToHost));
+    CUDA_TRY(cudaMemcpy(l, w.w.loss, sizeof(l), cudaMemcpyDeviceToHost));
     *loss = l[1] > 0 ? l[0] / l[1] : 0.0;
-    CUDA_TRY(cudaMemcpy(grads, w.grad.p, 4ull * emp::kMlpParams, cudaMemcpyDeviceToHost));
+    CUDA_TRY(cudaMemcpy(grads, w.w.grad, 4ull * emp::kMlpParams, cudaMemcpyDeviceToHost));
     return EMP_OK;
 }
 
@@ -439,7 +444,7 @@ extern "C" emp_status emp_mlp_train(emp_mlp model, const emp_puzzle* puzzles, ui
             CUDA_TRY(emp::mlp_adam_step(model->dev(), w.w.grad, model->m1.as<float>(), model->m2.as<float>(), lr,
                                         ++model->adam_steps, nullptr));
             double l[2];
-            CUDA_TRY(cudaMemcpy(l, w.loss.p, sizeof(l), cudaMemcpyDeviceToHost));
+            CUDA_TRY(cudaMemcpy(l, w.w.loss, sizeof(l), cudaMemcpyDeviceToHost));
             ep_loss += l[0];
             ep_w += l[1];
         }

@@ -89,8 +89,10 @@ struct MlpWork {
     float* dh2 = nullptr;   // [rows][256]
     float* dh1 = nullptr;   // [rows][256]
     float* grad = nullptr;  // kMlpParams
+    float* parts = nullptr; // mlp_part_floats(rows) partial sums of the gradient
     double* loss = nullptr; // [2]: weighted loss sum, weight sum
 };
+uint64_t mlp_part_floats(uint64_t n);
 // Forward of rows x[n][512] (f32) into h1, h2, s.
 cudaError_t mlp_forward_f32(const MlpDevice& m, const MlpWork& w, const float* x, uint64_t n, cudaStream_t stream);
 // Weighted logistic loss and its gradient with respect to every parameter (grad,
