@@ -20,9 +20,11 @@ uint64_t context_id()
         if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) != cudaSuccess) f = nullptr;
         return reinterpret_cast<Fn>(f);
     }();
-    cudaFree(nullptr);  // makes the device's primary context current
     unsigned long long id = 0;
-    return get && get(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+    if (!get) return 0;
+    if (get(nullptr, &id) == CUDA_SUCCESS) return id;
+    cudaFree(nullptr);  // makes the device's primary context current
+    return get(nullptr, &id) == CUDA_SUCCESS ? id : 0;
 }
 
 struct Pool {
@@ -82,8 +84,11 @@ cudaError_t device_alloc(void** out, size_t bytes, int* device, uint64_t* contex
                 cudaMemPoolTrimTo(p->pool, 0);
                 e = cudaMallocFromPoolAsync(out, bytes, p->pool, p->stream);
             }
-            // usable from any stream from here on
-            if (e == cudaSuccess) e = cudaStreamSynchronize(p->stream);
+            // usable from any stream from here on: nothing but the pool's own work is on its stream
+            if (e == cudaSuccess && cudaStreamQuery(p->stream) != cudaSuccess) {
+                cudaGetLastError();
+                e = cudaStreamSynchronize(p->stream);
+            }
             if (e == cudaSuccess) *context = id;
             return e;
         }
