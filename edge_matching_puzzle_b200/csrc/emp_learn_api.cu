@@ -236,12 +236,12 @@ extern "C" emp_status emp_mlp_score(emp_mlp model, const float* features, uint64
     EMP_TRY(use_device(model->device));
     DeviceBuffer x32, x16, s, err;
     CUDA_TRY(x32.alloc(4ull * emp::kMlpIn * n));
-    CUDA_TRY(x16.alloc(2ull * emp::kMlpIn * n));
+    CUDA_TRY(x16.alloc(emp::mlp_image_bytes(n)));
     CUDA_TRY(s.alloc(4ull * n));
     CUDA_TRY(err.alloc(sizeof(int)));
     CUDA_TRY(cudaMemset(err.p, 0, sizeof(int)));
     CUDA_TRY(cudaMemcpy(x32.p, features, 4ull * emp::kMlpIn * n, cudaMemcpyHostToDevice));
-    CUDA_TRY(emp::launch_f32_to_bf16(x32.as<float>(), x16.as<uint16_t>(), emp::kMlpIn * n, nullptr));
+    CUDA_TRY(emp::launch_rows_to_image(x32.as<float>(), x16.p, n, nullptr));
     CUDA_TRY(emp::launch_mlp_infer_tc(model->dev(), x16.p, n, s.as<float>(), err.as<int>(), nullptr));
     int e = 0;
     CUDA_TRY(cudaMemcpy(&e, err.p, sizeof(int), cudaMemcpyDeviceToHost));
@@ -496,7 +496,7 @@ extern "C" emp_status emp_bt_plan_order(emp_bt_plan plan, emp_mlp model)
     CUDA_TRY(d_score.alloc(4 * N));
     const uint64_t rows = std::min<uint64_t>(chunk, N) * per;
     CUDA_TRY(d_items.alloc(sizeof(emp::FeatItem) * rows));
-    CUDA_TRY(d_x.alloc(2ull * emp::kMlpIn * rows));
+    CUDA_TRY(d_x.alloc(emp::mlp_image_bytes(rows)));
     CUDA_TRY(d_s.alloc(4 * rows));
     CUDA_TRY(d_err.alloc(sizeof(int)));
     CUDA_TRY(cudaMemset(d_err.p, 0, sizeof(int)));

@@ -72,8 +72,9 @@ __device__ __forceinline__ uint32_t colour_edges(uint32_t cand, uint32_t c)
 }
 
 // ---------------------------------------------------------------------------
-// features: one warp per row; the lanes clear the row and count the colours of
-// the placed pieces, lane 0 sets the active entries
+// features: a warp takes eight rows and clears them, then four lanes a row count the colours of the
+// placed pieces and the first of them sets the active entries.  bf16 rows go straight into the
+// operand images of the inference (below), in which eight rows are whole lines.
 //
 //   [0, 128)    colour of each side of the oriented candidate (4 x 32 one-hot)
 //   [128, 140)  state of each side's neighbour: outside / placed / free (4 x 3)
@@ -83,21 +84,41 @@ __device__ __forceinline__ uint32_t colour_edges(uint32_t cand, uint32_t c)
 //   [252, 255)  kind: centre / border / corner
 //   255         constant 1
 //   [256, 512)  colours of the first two free sides, hashed (c1 * 32 + c2) mod 256
+// Operand images of the inference: row r of a tile of `rows` rows, element k, in chunks of
+// kKc elements of K, each in the canonical K-major layout without swizzle: 8-row x 16-byte core
+// matrices, K-adjacent ones 128 bytes apart, 8-row groups kKc * 16 bytes apart.
+constexpr uint32_t kKc = 64, kTileRows = 128;
+__device__ __forceinline__ uint32_t image_offset(uint32_t r, uint32_t k, uint32_t rows)
+{
+    return (k / kKc) * (rows * kKc * 2) + (r >> 3) * (kKc * 16) + ((k % kKc) >> 3) * 128 + (r & 7u) * 16 + (k & 7u) * 2;
+}
+constexpr uint32_t kXTileBytes = kTileRows * kMlpIn * 2;
+
 __global__ void features_kernel(const uint32_t* __restrict__ ftab, const unsigned long long* __restrict__ ftab_off,
                                 const FeatItem* __restrict__ items, uint64_t n, const uint16_t* __restrict__ prefixes,
-                                uint16_t* __restrict__ out_bf16, float* __restrict__ out_f32)
+                                uint8_t* __restrict__ image, float* __restrict__ out_f32)
 {
-    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t lane = threadIdx.x & 31u, sub = lane & 3u;
     const uint64_t nwarps = (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5;
-    for (uint64_t i = (blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x) >> 5; i < n; i += nwarps) {
-        if (out_bf16) {
-            uint4* row = reinterpret_cast<uint4*>(out_bf16 + i * kMlpIn);
-            row[lane] = make_uint4(0, 0, 0, 0);
-            row[lane + 32] = make_uint4(0, 0, 0, 0);
+    for (uint64_t g = (blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x) >> 5; g * 8 < n; g += nwarps) {
+        if (image) {
+            // the group's 1 KB in each chunk (rows past n belong to the last tile and are cleared too)
+            uint8_t* tile = image + (g / (kTileRows / 8)) * kXTileBytes;
+            const uint32_t off = static_cast<uint32_t>(g % (kTileRows / 8)) * (kKc * 16);
+            for (uint32_t c = 0; c < kMlpIn / kKc; ++c) {
+                uint4* q = reinterpret_cast<uint4*>(tile + c * (kTileRows * kKc * 2) + off);
+                q[lane] = make_uint4(0, 0, 0, 0);
+                q[lane + 32] = make_uint4(0, 0, 0, 0);
+            }
         } else {
-            uint4* row = reinterpret_cast<uint4*>(out_f32 + i * kMlpIn);
-            for (uint32_t j = 0; j < 4; ++j) row[lane + 32 * j] = make_uint4(0, 0, 0, 0);
+            for (uint64_t r = g * 8; r < g * 8 + 8 && r < n; ++r) {
+                uint4* row = reinterpret_cast<uint4*>(out_f32 + r * kMlpIn);
+                for (uint32_t j = 0; j < 4; ++j) row[lane + 32 * j] = make_uint4(0, 0, 0, 0);
+            }
         }
+        __syncwarp();
+        const bool mine = g * 8 + (lane >> 2) < n;
+        const uint64_t i = mine ? g * 8 + (lane >> 2) : n - 1;
         const FeatItem it = items[i];
         const uint32_t* T = ftab + ftab_off[it.puzzle];
         const uint32_t l = it.len, nlev = T[0];
@@ -110,40 +131,45 @@ __global__ void features_kernel(const uint32_t* __restrict__ ftab, const unsigne
         // edges of each free side's colour on the pieces placed before this level
         const uint16_t* pre = prefixes + it.prefix_off;
         uint32_t placed[4] = {0, 0, 0, 0};
-        for (uint32_t j = lane; j < l; j += 32) {
+        for (uint32_t j = sub; j < l; j += 4) {
             const uint32_t kj = (T[kFtLevelA + j] >> 8) & 0xFFu;
             const uint32_t cj = T[T[kFtKindOff + kj] + pre[j]];
             for (uint32_t s = 0; s < 4; ++s) placed[s] += colour_edges(cj, side_colour(cand, s));
         }
-        for (uint32_t s = 0; s < 4; ++s) placed[s] = __reduce_add_sync(kFull, placed[s]);
         __syncwarp();
-        if (lane == 0) {
-            uint32_t idx[24];
-            uint32_t k = 0;
-            uint32_t free_col[2];
-            uint32_t nfree = 0;
+        for (uint32_t s = 0; s < 4; ++s) {
+            placed[s] += __shfl_xor_sync(kFull, placed[s], 1);
+            placed[s] += __shfl_xor_sync(kFull, placed[s], 2);
+        }
+        if (mine && sub == 0) {
+            uint8_t* tile = image + (i / kTileRows) * kXTileBytes;
+            const uint32_t r = static_cast<uint32_t>(i % kTileRows);
+            auto set = [&](uint32_t k) {
+                if (image) *reinterpret_cast<uint16_t*>(tile + image_offset(r, k, kTileRows)) = 0x3F80u;  // bf16 1.0
+                else out_f32[i * kMlpIn + k] = 1.0f;
+            };
+            uint32_t free0 = 0, free1 = 0, nfree = 0;
+#pragma unroll
             for (uint32_t s = 0; s < 4; ++s) {
                 const uint32_t c = side_colour(cand, s);
-                idx[k++] = 32 * s + c;
+                set(32 * s + c);
                 const uint32_t state = nb[s] == 0xFFFFu ? 0u : (nb[s] < l ? 1u : 2u);
-                idx[k++] = 128 + 3 * s + state;
+                set(128 + 3 * s + state);
                 if (state == 2) {
                     const uint32_t left = T[kFtColours + c] - placed[s] - colour_edges(cand, c);
-                    idx[k++] = 140 + 16 * s + min(left, 15u);
-                    if (nfree < 2) free_col[nfree++] = c;
+                    set(140 + 16 * s + min(left, 15u));
+                    if (nfree == 0) free0 = c;
+                    if (nfree == 1) free1 = c;
+                    ++nfree;
                 }
             }
-            idx[k++] = 204 + x;
-            idx[k++] = 220 + y;
-            idx[k++] = 236 + min(l * 16 / max(nlev, 1u), 15u);
-            idx[k++] = 252 + min(kind, 2u);
-            idx[k++] = 255;
-            if (nfree == 2) idx[k++] = 256 + ((free_col[0] * 32 + free_col[1]) & 255u);
-            else if (nfree == 1) idx[k++] = 256 + free_col[0];
-            for (uint32_t j = 0; j < k; ++j) {
-                if (out_bf16) out_bf16[i * kMlpIn + idx[j]] = 0x3F80u;  // bf16 1.0
-                else out_f32[i * kMlpIn + idx[j]] = 1.0f;
-            }
+            set(204 + x);
+            set(220 + y);
+            set(236 + min(l * 16 / max(nlev, 1u), 15u));
+            set(252 + min(kind, 2u));
+            set(255);
+            if (nfree >= 2) set(256 + ((free0 * 32 + free1) & 255u));
+            else if (nfree == 1) set(256 + free0);
         }
         __syncwarp();
     }
@@ -152,24 +178,31 @@ __global__ void features_kernel(const uint32_t* __restrict__ ftab, const unsigne
 // ---------------------------------------------------------------------------
 // tensor-core inference
 //
-// One CTA (128 threads) scores 128 rows at a time:
-//   layer 1  D1[128 x 256] = X[128 x 512] . W1^T      4 chunks of K = 128
-//   layer 2  D2[128 x 256] = relu(D1 + b1) . W2^T     2 chunks of K = 128
+// One persistent CTA an SM scores 128 rows at a time:
+//   layer 1  D1[128 x 256] = X[128 x 512] . W1^T      8 chunks of K = 64
+//   layer 2  D2[128 x 256] = relu(D1 + b1) . W2^T     4 chunks of K = 64
 //   score    relu(D2 + b2) . w3 + b3                  in the epilogue
-// Operands sit in shared memory in the canonical K-major layout without
-// swizzle: 8-row x 16-byte core matrices, K-adjacent core matrices 128 bytes
-// apart (LBO), 8-row groups K*2*8 bytes apart (SBO).  Accumulators live in
-// tensor memory (512 columns: D1 in [0, 256), D2 in [256, 512)); thread 0
-// issues the MMAs, an mbarrier signalled by tcgen05.commit reports completion.
-constexpr uint32_t kTileRows = 128;
-constexpr uint32_t kChunk = 128;
-constexpr uint32_t kSmX = 0;                              // 128 x 128 bf16: 32 KB
-constexpr uint32_t kSmB = kSmX + kTileRows * kChunk * 2;  // 256 x 128 bf16: 64 KB
-constexpr uint32_t kSmH = kSmB + kMlpHidden * kChunk * 2; // 128 x 256 bf16: 64 KB
+// X, W1 and W2 lie in memory as operand images (image_offset), so a chunk is one or two bulk copies
+// into one of three stages.  One thread issues the copies, one the MMAs, and four warps read the
+// accumulators (tensor memory: D1 in columns [0, 256), D2 in [256, 512)), so that the copies run
+// ahead and the score of a tile overlaps layer 1 of the next.  tcgen05.commit frees stages and
+// reports accumulators.
+//
+// What bounds it: the bytes from L2 into an SM, 512 KB a tile (384 KB of weights), against 3072
+// cycles of MMA.  Measured on a B200, before (one warpgroup that staged chunks with plain loads
+// and waited for each) and after: 353 000 rows, 65 536 a launch, 2.04 ms -> 0.21 ms; a whole call
+// scoring 19 rows 107 us -> 81 us.
+constexpr uint32_t kStages = 3;
+constexpr uint32_t kXBytes = kTileRows * kKc * 2, kWBytes = kMlpHidden * kKc * 2;  // a chunk: 16 KB, 32 KB
+constexpr uint32_t kSmW = kXBytes, kStageBytes = kXBytes + kWBytes;
+constexpr uint32_t kSmH = kStages * kStageBytes;          // 128 x 256 bf16: 64 KB
 constexpr uint32_t kSmVec = kSmH + kTileRows * kMlpHidden * 2;  // b1, b2, w3 (f32)
 constexpr uint32_t kSmBar = kSmVec + 3 * kMlpHidden * 4;
-constexpr uint32_t kSmTotal = kSmBar + 16;
+enum : uint32_t { kBarFull = 0, kBarEmpty = kStages, kBarD1 = 2 * kStages, kBarH, kBarD2, kBarD2Free, kBarDrain, kBars };
+constexpr uint32_t kSmSlot = kSmBar + 8 * kBars;
+constexpr uint32_t kSmTotal = kSmSlot + 16;
 constexpr unsigned long long kWaitNs = 2000000000ull;     // 2 s per wait
+constexpr uint32_t kInferThreads = 192;                   // 4 epilogue warps, copies, MMAs
 
 // byte offset of element (r, k) in a K-major canonical tile whose rows hold kk elements
 __device__ __forceinline__ uint32_t canon(uint32_t r, uint32_t k, uint32_t kk)
@@ -240,40 +273,46 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v)
     for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
 }
 
-// copies rows [0, rows) x k-range [k0, k0 + kChunk) of a row-major bf16 matrix
-// (ld elements per row) into a canonical tile; rows >= valid are zero
-__device__ __forceinline__ void stage_chunk(uint8_t* dst, const uint16_t* src, uint32_t rows, uint64_t valid,
-                                            uint32_t ld, uint32_t k0)
+__device__ __forceinline__ void bar_init(uint32_t bar, uint32_t count)
 {
-    for (uint32_t p = threadIdx.x; p < rows * (kChunk / 8); p += blockDim.x) {
-        const uint32_t r = p / (kChunk / 8), kb = p % (kChunk / 8);
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (r < valid) v = *reinterpret_cast<const uint4*>(src + static_cast<uint64_t>(r) * ld + k0 + kb * 8);
-        *reinterpret_cast<uint4*>(dst + canon(r, kb * 8, kChunk)) = v;
-    }
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(uint32_t bar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void bar_expect(uint32_t bar, uint32_t bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
 }
 
-__global__ void __launch_bounds__(128, 1)
-    mlp_infer_kernel(const uint16_t* __restrict__ x, uint64_t n, const uint16_t* __restrict__ w1,
-                     const uint16_t* __restrict__ w2, const float* __restrict__ params, float* __restrict__ out,
+__global__ void __launch_bounds__(kInferThreads, 1)
+    mlp_infer_kernel(const uint8_t* __restrict__ x, uint64_t n, const uint8_t* __restrict__ w1,
+                     const uint8_t* __restrict__ w2, const float* __restrict__ params, float* __restrict__ out,
                      int* err)
 {
     extern __shared__ __align__(1024) uint8_t sm[];
     const uint32_t tid = threadIdx.x, warp = tid >> 5;
     const uint32_t base = static_cast<uint32_t>(__cvta_generic_to_shared(sm));
-    const uint32_t bar = base + kSmBar;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + kSmBar + 8);
+    auto bar = [&](uint32_t k) { return base + kSmBar + 8 * k; };
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + kSmSlot);
     float* vb1 = reinterpret_cast<float*>(sm + kSmVec);
     float* vb2 = vb1 + kMlpHidden;
     float* vw3 = vb2 + kMlpHidden;
-    for (uint32_t j = tid; j < kMlpHidden; j += blockDim.x) {
+    for (uint32_t j = tid; j < kMlpHidden; j += kInferThreads) {
         vb1[j] = params[kOffB1 + j];
         vb2[j] = params[kOffB2 + j];
         vw3[j] = params[kOffW3 + j];
     }
     const float b3 = params[kOffB3];
     if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+        for (uint32_t k = 0; k < kBars; ++k) bar_init(bar(k), k == kBarH || k == kBarD2Free ? 128u : 1u);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -286,88 +325,113 @@ __global__ void __launch_bounds__(128, 1)
     fence_after();
     const uint32_t tmem = *tmem_slot;
     const uint32_t d1 = tmem, d2 = tmem + kMlpHidden;
-    const uint32_t lane_base = (32u * (warp & 3u)) << 16;  // this warp's 32 tensor-memory lanes
-    uint32_t phase = 0;
-    bool failed = false;
     const uint64_t tiles = (n + kTileRows - 1) / kTileRows;
+    constexpr uint32_t kC1 = kMlpIn / kKc, kC2 = kMlpHidden / kKc;
+    bool ok = true;
+    uint32_t issued = 0;  // copy thread: chunks whose copies were issued
 
-    for (uint64_t tile = blockIdx.x; tile < tiles && !failed; tile += gridDim.x) {
-        const uint64_t row0 = tile * kTileRows;
-        const uint64_t valid = n - row0 < kTileRows ? n - row0 : kTileRows;
-        // ---- layer 1 ----
-        for (uint32_t c = 0; c < kMlpIn / kChunk && !failed; ++c) {
-            stage_chunk(sm + kSmX, x + row0 * kMlpIn, kTileRows, valid, kMlpIn, c * kChunk);
-            stage_chunk(sm + kSmB, w1, kMlpHidden, kMlpHidden, kMlpIn, c * kChunk);
+    if (warp == 4 && (tid & 31u) == 0) {
+        // ---- copies: a tile's chunks of X and W1, then of W2 ----
+        for (uint64_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+            for (uint32_t c = 0; c < kC1 + kC2 && ok; ++c) {
+                const uint32_t s = issued % kStages;
+                ok = bar_wait(bar(kBarEmpty + s), ((issued / kStages) & 1u) ^ 1u);
+                if (!ok) break;
+                const uint32_t dst = base + s * kStageBytes, full = bar(kBarFull + s);
+                if (c < kC1) {
+                    bar_expect(full, kXBytes + kWBytes);
+                    bulk_copy(dst, x + tile * kXTileBytes + c * kXBytes, kXBytes, full);
+                    bulk_copy(dst + kSmW, w1 + c * kWBytes, kWBytes, full);
+                } else {
+                    bar_expect(full, kWBytes);
+                    bulk_copy(dst + kSmW, w2 + (c - kC1) * kWBytes, kWBytes, full);
+                }
+                ++issued;
+            }
+        }
+        // copies in flight have landed before the CTA's shared memory goes away
+        for (uint32_t k = issued > kStages ? issued - kStages : 0; k < issued; ++k)
+            bar_wait(bar(kBarFull + k % kStages), (k / kStages) & 1u);
+    } else if (warp == 5 && (tid & 31u) == 0) {
+        // ---- MMAs ----
+        uint32_t k = 0, t = 0;  // chunks and tiles so far
+        for (uint64_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++t) {
+            // D1 is free: the epilogue has read it when it hands over H
+            if (t) ok = bar_wait(bar(kBarH), (t - 1) & 1u);
+            for (uint32_t c = 0; c < kC1 + kC2 && ok; ++c, ++k) {
+                if (c == kC1) {
+                    mma_commit(bar(kBarD1));
+                    ok = bar_wait(bar(kBarH), t & 1u);  // relu(D1 + b1) is in shared memory
+                    if (ok && t) ok = bar_wait(bar(kBarD2Free), (t - 1) & 1u);
+                    if (!ok) break;
+                }
+                const uint32_t s = k % kStages;
+                ok = bar_wait(bar(kBarFull + s), (k / kStages) & 1u);
+                if (!ok) break;
+                fence_after();
+                const uint32_t at = base + s * kStageBytes;
+                for (uint32_t kk = 0; kk < kKc / 16; ++kk) {
+                    const uint64_t b = smem_desc(at + kSmW + kk * 256, 128, kKc * 16);
+                    if (c < kC1)
+                        mma_bf16(d1, smem_desc(at + kk * 256, 128, kKc * 16), b, (c | kk) != 0);
+                    else
+                        mma_bf16(d2, smem_desc(base + kSmH + ((c - kC1) * (kKc / 8) + kk * 2) * 128, 128, kMlpHidden * 16),
+                                 b, ((c - kC1) | kk) != 0);
+                }
+                mma_commit(bar(kBarEmpty + s));
+            }
+            if (ok) mma_commit(bar(kBarD2));
+        }
+        // MMAs in flight have ended before tensor memory is freed
+        mma_commit(bar(kBarDrain));
+        bar_wait(bar(kBarDrain), 0);
+    } else if (warp < 4) {
+        // ---- epilogues: this thread's row is its tensor-memory lane ----
+        const uint32_t lane_base = (32u * warp) << 16, r = tid;
+        uint32_t t = 0;
+        for (uint64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++t) {
+            ok = bar_wait(bar(kBarD1), t & 1u);
+            if (!__all_sync(kFull, ok)) break;
+            fence_after();
+            // bias, relu, bf16 into the layer-2 operand (layer 2 of the tile before has ended: its score
+            // was taken)
+            for (uint32_t c0 = 0; c0 < kMlpHidden; c0 += 32) {
+                float v[32];
+                tmem_ld32(d1 + lane_base + c0, v);
+                for (uint32_t g = 0; g < 4; ++g) {
+                    uint32_t w[4];
+                    for (uint32_t h = 0; h < 4; ++h) {
+                        const uint32_t j = c0 + g * 8 + 2 * h;
+                        const __nv_bfloat162 pr = __floats2bfloat162_rn(fmaxf(v[g * 8 + 2 * h] + vb1[j], 0.f),
+                                                                        fmaxf(v[g * 8 + 2 * h + 1] + vb1[j + 1], 0.f));
+                        w[h] = *reinterpret_cast<const uint32_t*>(&pr);
+                    }
+                    *reinterpret_cast<uint4*>(sm + kSmH + canon(r, c0 + g * 8, kMlpHidden)) =
+                        make_uint4(w[0], w[1], w[2], w[3]);
+                }
+            }
             fence_proxy_async();
             fence_before();
-            __syncthreads();
-            if (tid == 0) {
-                fence_after();
-                for (uint32_t kk = 0; kk < kChunk / 16; ++kk) {
-                    const uint64_t a = smem_desc(base + kSmX + kk * 256, 128, kChunk * 16);
-                    const uint64_t b = smem_desc(base + kSmB + kk * 256, 128, kChunk * 16);
-                    mma_bf16(d1, a, b, (c | kk) != 0);
-                }
-                mma_commit(bar);
-            }
-            failed = __syncthreads_or(!bar_wait(bar, phase));
-            phase ^= 1u;
+            bar_arrive(bar(kBarH));
+            ok = bar_wait(bar(kBarD2), t & 1u);
+            if (!__all_sync(kFull, ok)) break;
             fence_after();
-        }
-        if (failed) break;
-        // ---- epilogue 1: bias, relu, bf16 into the layer-2 operand ----
-        const uint32_t r = tid;  // this thread's row = its tensor-memory lane
-        for (uint32_t c0 = 0; c0 < kMlpHidden; c0 += 32) {
-            float v[32];
-            tmem_ld32(d1 + lane_base + c0, v);
-            for (uint32_t g = 0; g < 4; ++g) {
-                uint32_t w[4];
-                for (uint32_t h = 0; h < 4; ++h) {
-                    const uint32_t j = c0 + g * 8 + 2 * h;
-                    const __nv_bfloat162 pr =
-                        __floats2bfloat162_rn(fmaxf(v[g * 8 + 2 * h] + vb1[j], 0.f), fmaxf(v[g * 8 + 2 * h + 1] + vb1[j + 1], 0.f));
-                    w[h] = *reinterpret_cast<const uint32_t*>(&pr);
-                }
-                *reinterpret_cast<uint4*>(sm + kSmH + canon(r, c0 + g * 8, kMlpHidden)) = make_uint4(w[0], w[1], w[2], w[3]);
-            }
-        }
-        fence_proxy_async();
-        // ---- layer 2 ----
-        for (uint32_t c = 0; c < kMlpHidden / kChunk && !failed; ++c) {
-            stage_chunk(sm + kSmB, w2, kMlpHidden, kMlpHidden, kMlpHidden, c * kChunk);
-            fence_proxy_async();
-            fence_before();
-            __syncthreads();
-            if (tid == 0) {
-                fence_after();
-                for (uint32_t kk = 0; kk < kChunk / 16; ++kk) {
-                    const uint64_t a = smem_desc(base + kSmH + (c * kChunk / 8 + kk * 2) * 128, 128, kMlpHidden * 16);
-                    const uint64_t b = smem_desc(base + kSmB + kk * 256, 128, kChunk * 16);
-                    mma_bf16(d2, a, b, (c | kk) != 0);
-                }
-                mma_commit(bar);
-            }
-            failed = __syncthreads_or(!bar_wait(bar, phase));
-            phase ^= 1u;
-            fence_after();
-        }
-        if (failed) break;
-        // ---- epilogue 2: bias, relu, dot with w3 ----
-        float score = b3;
-        for (uint32_t c0 = 0; c0 < kMlpHidden; c0 += 32) {
-            float v[32];
-            tmem_ld32(d2 + lane_base + c0, v);
+            // bias, relu, dot with w3
+            float score = b3;
+            for (uint32_t c0 = 0; c0 < kMlpHidden; c0 += 32) {
+                float v[32];
+                tmem_ld32(d2 + lane_base + c0, v);
 #pragma unroll
-            for (int j = 0; j < 32; ++j) score += fmaxf(v[j] + vb2[c0 + j], 0.f) * vw3[c0 + j];
+                for (int j = 0; j < 32; ++j) score += fmaxf(v[j] + vb2[c0 + j], 0.f) * vw3[c0 + j];
+            }
+            fence_before();
+            bar_arrive(bar(kBarD2Free));
+            const uint64_t row = tile * kTileRows + r;
+            if (row < n) out[row] = score;
         }
-        if (r < valid) out[row0 + r] = score;
-        fence_before();
-        __syncthreads();
     }
-    if (failed) {
-        if (tid == 0) atomicExch(err, 1);
-        bar_wait(bar, phase ^ 1u);  // the phase that timed out: let its MMAs finish (bounded) before freeing
-    }
+    if (!ok) atomicExch(err, 1);
+    __syncwarp();
     fence_before();
     __syncthreads();
     if (warp == 0) {
@@ -632,12 +696,11 @@ __global__ void adam_kernel(float* p, const float* __restrict__ g, float* m1, fl
     }
 }
 
-__global__ void pack_bf16_kernel(const float* __restrict__ src, uint16_t* __restrict__ dst, uint32_t n)
+// a weight matrix (rows x cols, row-major) into its operand image
+__global__ void pack_bf16_kernel(const float* __restrict__ src, uint8_t* __restrict__ dst, uint32_t rows, uint32_t cols)
 {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const __nv_bfloat16 v = __float2bfloat16_rn(src[i]);
-        dst[i] = *reinterpret_cast<const uint16_t*>(&v);
-    }
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < rows * cols; i += gridDim.x * blockDim.x)
+        *reinterpret_cast<__nv_bfloat16*>(dst + image_offset(i / cols, i % cols, rows)) = __float2bfloat16_rn(src[i]);
 }
 
 uint32_t grid_for(uint64_t n, uint32_t threads)
@@ -645,12 +708,23 @@ uint32_t grid_for(uint64_t n, uint32_t threads)
     return static_cast<uint32_t>(std::min<uint64_t>((n + threads - 1) / threads, 148ull * 16));
 }
 
-__global__ void f32_to_bf16_kernel(const float* __restrict__ src, uint16_t* __restrict__ dst, uint64_t n)
+// f32 feature rows into operand images; eight lanes write one line of eight rows' 16 bytes
+__global__ void rows_to_image_kernel(const float* __restrict__ src, uint8_t* __restrict__ image, uint64_t n)
 {
-    for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < n;
+    constexpr uint32_t kPieces = kMlpIn / 8;
+    const uint64_t total = (n + 7) / 8 * 8 * kPieces;
+    for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < total;
          i += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
-        const __nv_bfloat16 v = __float2bfloat16_rn(src[i]);
-        dst[i] = *reinterpret_cast<const uint16_t*>(&v);
+        const uint64_t row = i / (8 * kPieces) * 8 + (i & 7u);
+        const uint32_t k = static_cast<uint32_t>(i / 8 % kPieces) * 8;
+        if (row >= n) continue;
+        const float4 a = *reinterpret_cast<const float4*>(src + row * kMlpIn + k);
+        const float4 b = *reinterpret_cast<const float4*>(src + row * kMlpIn + k + 4);
+        const __nv_bfloat162 p[4] = {__floats2bfloat162_rn(a.x, a.y), __floats2bfloat162_rn(a.z, a.w),
+                                     __floats2bfloat162_rn(b.x, b.y), __floats2bfloat162_rn(b.z, b.w)};
+        *reinterpret_cast<uint4*>(image + (row / kTileRows) * kXTileBytes +
+                                  image_offset(static_cast<uint32_t>(row % kTileRows), k, kTileRows)) =
+            *reinterpret_cast<const uint4*>(p);
     }
 }
 
@@ -717,10 +791,13 @@ __global__ void order_accumulate_kernel(const float* __restrict__ scores, const 
 
 }  // namespace
 
-cudaError_t launch_f32_to_bf16(const float* src, uint16_t* dst, uint64_t n, cudaStream_t stream)
+uint64_t mlp_image_bytes(uint64_t n) { return (n + kTileRows - 1) / kTileRows * kXTileBytes; }
+
+cudaError_t launch_rows_to_image(const float* src, void* image, uint64_t n, cudaStream_t stream)
 {
     if (!n) return cudaSuccess;
-    f32_to_bf16_kernel<<<grid_for(n, 256), 256, 0, stream>>>(src, dst, n);
+    rows_to_image_kernel<<<grid_for((n + 7) / 8 * 8 * (kMlpIn / 8), 256), 256, 0, stream>>>(
+        src, static_cast<uint8_t*>(image), n);
     return cudaGetLastError();
 }
 
@@ -750,25 +827,27 @@ cudaError_t launch_order_accumulate(const float* scores, const FeatItem* items, 
 }
 
 cudaError_t launch_features(const uint32_t* ftab, const unsigned long long* ftab_off, const FeatItem* items,
-                            uint64_t n, const uint16_t* prefixes, void* out_bf16, float* out_f32, cudaStream_t stream)
+                            uint64_t n, const uint16_t* prefixes, void* image, float* out_f32, cudaStream_t stream)
 {
     if (!n) return cudaSuccess;
-    const uint64_t blocks = std::min<uint64_t>((n + 7) / 8, 148ull * 32);  // 8 warps (rows) per block
-    features_kernel<<<static_cast<uint32_t>(blocks), 256, 0, stream>>>(
-        ftab, ftab_off, items, n, prefixes, static_cast<uint16_t*>(out_bf16), out_f32);
+    const uint64_t blocks = std::min<uint64_t>((n + 31) / 32, 148ull * 64);  // 4 warps of eight rows
+    features_kernel<<<static_cast<uint32_t>(blocks), 128, 0, stream>>>(
+        ftab, ftab_off, items, n, prefixes, static_cast<uint8_t*>(image), out_f32);
     return cudaGetLastError();
 }
 
 cudaError_t launch_mlp_pack_bf16(const MlpDevice& m, cudaStream_t stream)
 {
-    pack_bf16_kernel<<<256, 256, 0, stream>>>(m.params + kOffW1, m.w1_bf16, kMlpHidden * kMlpIn);
-    pack_bf16_kernel<<<256, 256, 0, stream>>>(m.params + kOffW2, m.w2_bf16, kMlpHidden * kMlpHidden);
+    pack_bf16_kernel<<<256, 256, 0, stream>>>(m.params + kOffW1, reinterpret_cast<uint8_t*>(m.w1_bf16), kMlpHidden,
+                                              kMlpIn);
+    pack_bf16_kernel<<<256, 256, 0, stream>>>(m.params + kOffW2, reinterpret_cast<uint8_t*>(m.w2_bf16), kMlpHidden,
+                                              kMlpHidden);
     return cudaGetLastError();
 }
 
 size_t mlp_infer_smem_bytes() { return kSmTotal; }
 
-cudaError_t launch_mlp_infer_tc(const MlpDevice& m, const void* x_bf16, uint64_t n, float* scores, int* err,
+cudaError_t launch_mlp_infer_tc(const MlpDevice& m, const void* image, uint64_t n, float* scores, int* err,
                                 cudaStream_t stream)
 {
     if (!n) return cudaSuccess;
@@ -780,8 +859,9 @@ cudaError_t launch_mlp_infer_tc(const MlpDevice& m, const void* x_bf16, uint64_t
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const uint64_t tiles = (n + kTileRows - 1) / kTileRows;
     const uint32_t grid = static_cast<uint32_t>(std::min<uint64_t>(tiles, static_cast<uint64_t>(sms)));
-    mlp_infer_kernel<<<grid, 128, kSmTotal, stream>>>(static_cast<const uint16_t*>(x_bf16), n, m.w1_bf16, m.w2_bf16,
-                                                      m.params, scores, err);
+    mlp_infer_kernel<<<grid, kInferThreads, kSmTotal, stream>>>(
+        static_cast<const uint8_t*>(image), n, reinterpret_cast<const uint8_t*>(m.w1_bf16),
+        reinterpret_cast<const uint8_t*>(m.w2_bf16), m.params, scores, err);
     return cudaGetLastError();
 }
 

@@ -47,21 +47,23 @@ struct FeatItem {
     uint16_t t;
 };
 
-// Feature rows (kMlpIn values each) as bf16 (inference) or f32 (training): one
-// of out_bf16 / out_f32 is null.
+// Feature rows (kMlpIn values each) as bf16 in operand images (inference, mlp_image_bytes(n)
+// bytes) or as f32 rows (training): one of image / out_f32 is null.
 cudaError_t launch_features(const uint32_t* ftab, const unsigned long long* ftab_off, const FeatItem* items,
-                            uint64_t n, const uint16_t* prefixes, void* out_bf16, float* out_f32,
+                            uint64_t n, const uint16_t* prefixes, void* image, float* out_f32,
                             cudaStream_t stream);
 
-// Device copy of the network: f32 master parameters and the bf16 operands of the
-// tensor-core inference (W1 and W2 as stored, K-major).
+// Device copy of the network: f32 master parameters and the bf16 operand images of the
+// tensor-core inference.
 struct MlpDevice {
     float* params = nullptr;        // kMlpParams
-    uint16_t* w1_bf16 = nullptr;    // [256][512]
-    uint16_t* w2_bf16 = nullptr;    // [256][256]
+    uint16_t* w1_bf16 = nullptr;    // 256 x 512
+    uint16_t* w2_bf16 = nullptr;    // 256 x 256
 };
 cudaError_t launch_mlp_pack_bf16(const MlpDevice& m, cudaStream_t stream);
-cudaError_t launch_f32_to_bf16(const float* src, uint16_t* dst, uint64_t n, cudaStream_t stream);
+// Bytes of the operand images of n feature rows (tiles of 128 rows), and f32 rows into them.
+uint64_t mlp_image_bytes(uint64_t n);
+cudaError_t launch_rows_to_image(const float* src, void* image, uint64_t n, cudaStream_t stream);
 // rows[i] = src[idx[i]] for rows of `cols` floats, and the per-row values y, w
 cudaError_t launch_gather_rows(const float* src, const uint32_t* idx, uint64_t n, uint32_t cols, float* dst,
                                const float* y, const float* w, float* y_out, float* w_out, cudaStream_t stream);
@@ -72,10 +74,10 @@ cudaError_t launch_order_items(const uint16_t* prefixes, const uint32_t* prefix_
 cudaError_t launch_order_accumulate(const float* scores, const FeatItem* items, uint64_t count, uint32_t depth,
                                     float* prefix_score, cudaStream_t stream);
 
-// Scores of n feature rows (bf16, row-major [n][512]) with the tensor cores
+// Scores of n feature rows (bf16 operand images) with the tensor cores
 // (tcgen05, BF16 operands, FP32 accumulation in tensor memory).  err receives a
 // nonzero code when a wait inside the kernel ran out of time.
-cudaError_t launch_mlp_infer_tc(const MlpDevice& m, const void* x_bf16, uint64_t n, float* scores, int* err,
+cudaError_t launch_mlp_infer_tc(const MlpDevice& m, const void* image, uint64_t n, float* scores, int* err,
                                 cudaStream_t stream);
 size_t mlp_infer_smem_bytes();
 
