@@ -24,7 +24,9 @@
 // What bounds it: instruction issue (74 % of the slots in the main rounds on a B200, 24 warps
 // an SM, shared-memory latency behind them); 30 of 32 lanes have work at a step, 22 of them a
 // candidate.  Measured, 1/64 of the 8x8 tree of 4 border / 8 interior colours, seed 0
-// (2.77e9 placements): 62.9 ms with dfs_kernel (4.4e10 placements/s), 26.3 ms here (1.05e11/s).
+// (2.77e9 placements): 62.9 ms with dfs_kernel (4.4e10 placements/s), 25.7 ms here (1.08e11/s).
+// The step with selects in place of its two divergent regions took 27.6 ms, with the sharing
+// inside a warp inlined 26.1 ms (registers).
 #include "emp_bt.h"
 
 #include <cuda_runtime.h>
@@ -62,7 +64,7 @@ __device__ __forceinline__ uint64_t ldg64(const uint32_t* p)
 
 template <int NW>
 struct Search {
-    uint64_t orig, nodes, sols, steps;
+    uint64_t orig, nodes, sols;
     const uint32_t* tb;              // the puzzle's blob
     uint32_t pz, n, L, base, space;
     int row;                         // byte offset of level L's row
@@ -135,7 +137,7 @@ __device__ __forceinline__ uint32_t word_space(uint32_t w) { return (w >> 17) & 
 __device__ __forceinline__ int word_row(uint32_t w) { return static_cast<int>((w >> 14) & 0x3FFF0u); }
 __device__ __forceinline__ uint32_t make_word(uint32_t e, uint32_t slot, bool more, uint32_t space, int row)
 {
-    return ((e >> 9) & 31u) | (slot << 8) | (static_cast<uint32_t>(more) << 16) | (space << 17) |
+    return (e >> 9) | (slot << 8) | (static_cast<uint32_t>(more) << 16) | (space << 17) |
            (static_cast<uint32_t>(row) << 14);
 }
 // byte offset of the row at a level with descriptor d: west entry and north colour
@@ -241,11 +243,11 @@ __device__ __forceinline__ void level_candidates(Search<NW>& s)
     if (static_cast<int64_t>(r.m[NW - 1]) < 0) only_tried<NW>(s.tb + r.clears, s.R);
 }
 
-// whether the trials of the candidates r of a row have to be replayed
+// whether a row's trials have to be replayed
 template <int NW>
-__device__ __forceinline__ bool flagged(const Row<NW>& row, const uint64_t* r)
+__device__ __forceinline__ bool flagged(const Row<NW>& row)
 {
-    return static_cast<int64_t>(row.m[NW - 1]) < 0 && (NW > 1 || (r[0] & (r[0] - 1)) != 0);
+    return static_cast<int64_t>(row.m[NW - 1]) < 0;
 }
 
 // of those, the ones above a slot
@@ -270,7 +272,7 @@ __device__ __forceinline__ uint32_t word_transition(const Search<NW>& s, uint32_
     uint32_t ki = __ldg(reinterpret_cast<const uint8_t*>(tb + __ldg(tb + 9)) + space * 64 * NW + slot);
     const uint32_t nborder = __ldg(tb + 11);
     if (space && ki >= nborder) ki -= nborder;
-    return (ki << 2) | (Tab<SM, NW>::entry(s, Tab<SM, NW>::row(s, word_row(word)).entries, slot) >> 14);
+    return (ki << 2) | (Tab<SM, NW>::entry(s, Tab<SM, NW>::row(s, word_row(word)).entries, slot) & 3u);
 }
 
 // (The functions below that are not inlined take the state by value: a reference would keep
@@ -292,7 +294,6 @@ __device__ __forceinline__ void start_search(Search<NW>& s, uint32_t len)
     s.base = len;
     s.nodes = 0;
     s.sols = 0;
-    s.steps = 0;
     s.active = true;
 }
 
@@ -323,38 +324,35 @@ __device__ __forceinline__ void load_item(const BtLaunch& P, Search<NW>& s, cons
         s.O[w] = w ? 0ull : g.z | static_cast<uint64_t>(g.w) << 32;
     }
     s.row = static_cast<int>(g.x);
-    SlotBits bits{0ull, 0ull};
-    uint32_t from = 0;               // the slot placed at the level
-    const bool resumed = len < h.z;  // else the state's own level, from its first slot left
-    const uint32_t* pre = st + state_header(NW);
-    for (uint32_t l = 0; l < h.z; l += 4) {
-        const uint4 v = *reinterpret_cast<const uint4*>(pre + l);
-        const uint32_t word[4] = {v.x, v.y, v.z, v.w};
+    // the whole stack first, four loads of four words on their way at a time ...
+    const uint4* pre = reinterpret_cast<const uint4*>(st + state_header(NW));
+    for (uint32_t l = 0; l < h.z; l += 16) {
+        uint4 v[4];
 #pragma unroll
-        for (uint32_t j = 0; j < 4; ++j) {
-            if (l + j < len) {
-                stk[(l + j) * T] = word[j];
-            } else if (l + j < h.z) {
-                // a piece at or past the level is given back
-                const uint32_t slot = word_slot(word[j]);
-                const SlotBits q = Tab<SM, NW>::slot(P, s, word_space(word[j]), slot);
-                to_space<NW>(s, word_space(word[j]));
-                toggle<NW>(s.A, slot, q.toggle);
-                if (l + j == len) {
-                    s.row = word_row(word[j]);
-                    from = slot;
-                    bits = q;
-                }
+        for (uint32_t j = 0; j < 4; ++j)
+            if (l + 4 * j < h.z) v[j] = pre[l / 4 + j];
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j)
+            if (l + 4 * j < h.z) {
+                uint32_t* q = stk + (l + 4 * j) * T;
+                q[0] = v[j].x;
+                q[T] = v[j].y;
+                q[2 * T] = v[j].z;
+                q[3 * T] = v[j].w;
             }
-        }
+    }
+    // ... then the pieces at and past the level are given back
+    for (uint32_t l = len; l < h.z; ++l) {
+        const uint32_t word = stk[l * T], slot = word_slot(word);
+        to_space<NW>(s, word_space(word));
+        toggle<NW>(s.A, slot, Tab<SM, NW>::slot(P, s, word_space(word), slot).toggle);
     }
     to_space<NW>(s, desc_space(Tab<SM, NW>::desc(s, len)));
+    if (len < h.z) s.row = word_row(stk[len * T]);
     level_candidates<SM, NW>(s);
-    if (resumed) {
-        above_slot<NW>(s.R, from, bits.above);
-    } else if (g.y) {
-        above_slot<NW>(s.R, g.y - 1, Tab<SM, NW>::slot(P, s, s.space, g.y - 1).above);
-    }
+    // after the piece placed at the level, or from the first slot left at the state's own level
+    const uint32_t from = len < h.z ? word_slot(stk[len * T]) + 1 : g.y;
+    if (from) above_slot<NW>(s.R, from - 1, Tab<SM, NW>::slot(P, s, s.space, from - 1).above);
     start_search<NW>(s, len);
 }
 
@@ -388,7 +386,7 @@ __device__ __forceinline__ void load_record(const BtLaunch& P, Search<NW>& s, co
         const int entries = Tab<SM, NW>::row(s, s.row).entries;
         uint32_t e = Tab<SM, NW>::entry(s, entries, slot);
         // the piece's slots in this row ascend with the orientation
-        for (int k = 0; k < 3 && (e >> 14) != (t & 3u); ++k) e = Tab<SM, NW>::entry(s, entries, ++slot);
+        for (int k = 0; k < 3 && (e & 3u) != (t & 3u); ++k) e = Tab<SM, NW>::entry(s, entries, ++slot);
         toggle<NW>(s.A, slot, Tab<SM, NW>::slot(P, s, s.space, slot).toggle);
         stk[l * T] = make_word(e, slot, false, s.space, s.row);
         west = e;
@@ -513,8 +511,75 @@ __device__ __noinline__ bool split_state(const BtLaunch& P, uint32_t* out, const
     return true;
 }
 
-// Persistent search over the records of a round; the fetch, the hand-back rule and the
-// checks of the deadline, cancellation and stop-at-first flags are those of dfs_kernel.
+// Once a round's queue is empty, idle lanes of a warp take work from its busy ones: the rest of
+// their shallowest open level.  The thief copies the path down to that level and gives back, in
+// its copy of the availability, the pieces from there on; the donor, all of whose shallower
+// levels are exhausted, ends its search above that level.  Measured on a B200 (split budget 64
+// without sharing, 256 with it): a 7x7 count of 2.3e6 placements 0.56 ms in 13 rounds -> 0.37 ms
+// in 5; 1/1024 of the tree above 3.84 -> 3.43 ms, 1/64 25.3 -> 25.7 ms at the same 30 -> 16 rounds.
+template <bool SM, int NW, int T>
+__device__ __noinline__ Search<NW> share_in_warp(const BtLaunch& P, Search<NW> s, uint32_t* stk)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t open = ~0u;
+    if (s.active)
+        for (uint32_t l = s.base; l < s.L; ++l)
+            if (word_more(stk[l * T])) {
+                open = l;
+                break;
+            }
+    __syncwarp();
+    const unsigned donors = __ballot_sync(kFull, open != ~0u), idle = __ballot_sync(kFull, !s.active);
+    if (!donors) return s;
+    const uint32_t lt = (1u << lane) - 1u;
+    const bool thief = !s.active && __popc(idle & lt) < __popc(donors);
+    const bool donor = open != ~0u && __popc(donors & lt) < __popc(idle);
+    const uint32_t from = thief ? __fns(donors, 0, __popc(idle & lt) + 1) : lane;
+    const uint32_t level = __shfl_sync(kFull, open, from), top = __shfl_sync(kFull, s.L, from);
+    const uint32_t space = __shfl_sync(kFull, s.space, from), pz = __shfl_sync(kFull, s.pz, from);
+    const uint64_t orig = __shfl_sync(kFull, s.orig, from);
+    uint64_t a[NW], o[NW];
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+        a[w] = __shfl_sync(kFull, s.A[w], from);
+        o[w] = __shfl_sync(kFull, s.O[w], from);
+    }
+    if (thief) {
+        const uint32_t* col = stk + static_cast<int>(from) - static_cast<int>(lane);
+        s.orig = orig;
+        start_puzzle<SM, NW>(P, s, pz);
+        s.space = space;
+#pragma unroll
+        for (int w = 0; w < NW; ++w) {
+            s.A[w] = a[w];
+            s.O[w] = o[w];
+        }
+#pragma unroll 4
+        for (uint32_t l = 0; l < level; ++l) stk[l * T] = col[l * T];
+        for (uint32_t l = level; l < top; ++l) {
+            const uint32_t word = col[l * T], slot = word_slot(word);
+            to_space<NW>(s, word_space(word));
+            toggle<NW>(s.A, slot, Tab<SM, NW>::slot(P, s, word_space(word), slot).toggle);
+        }
+        const uint32_t word = col[level * T], slot = word_slot(word);
+        to_space<NW>(s, word_space(word));
+        s.row = word_row(word);
+        level_candidates<SM, NW>(s);
+        above_slot<NW>(s.R, slot, Tab<SM, NW>::slot(P, s, s.space, slot).above);
+        start_search<NW>(s, level);
+    }
+    __syncwarp();
+    if (donor) {
+        stk[open * T] &= ~(1u << 16);
+        s.base = open + 1;
+    }
+    __syncwarp();
+    return s;
+}
+
+// Persistent search over the records of a round; the fetch and the checks of the deadline,
+// cancellation and stop-at-first flags are those of dfs_kernel.  Work goes back to the queue for
+// the next round once a warp has searched on for the split budget after the queue ran empty.
 template <int NW, bool SM, bool GS, int T, int kStepsPerFetch>
 __global__ void __launch_bounds__(T, (NW == 1 && SM ? 768 : 512) / T) dfs_compact_kernel(const __grid_constant__ BtLaunch P)
 {
@@ -533,6 +598,8 @@ __global__ void __launch_bounds__(T, (NW == 1 && SM ? 768 : 512) / T) dfs_compac
     bool alive = true;
     bool drained = false;      // warp-uniform: the input queue of this round is empty
     uint32_t iteration = 0;    // warp-uniform loop counter
+    uint32_t alone = 0;        // warp-uniform: steps since the warp found the queue empty (no more
+                               // than it takes to compare)
     uint32_t since_check = 0;  // steps since the last look at the global flags
     const uint64_t deadline = *(volatile unsigned long long*)&P.ctl->deadline;
     const uint64_t n_in = P.n_in_from_ctl ? *(volatile unsigned long long*)&P.ctl->n_in : P.n_in;
@@ -554,6 +621,7 @@ __global__ void __launch_bounds__(T, (NW == 1 && SM ? 768 : 512) / T) dfs_compac
 
     for (;; ++iteration) {
         // ---- work fetch: one atomic per warp, ranks from the ballot ----
+        if (drained && !s.active) alive = false;
         const bool need = alive && !s.active;
         const unsigned needmask = __ballot_sync(kFull, need);
         if (needmask) {
@@ -588,6 +656,13 @@ __global__ void __launch_bounds__(T, (NW == 1 && SM ? 768 : 512) / T) dfs_compac
             c = __shfl_sync(kFull, c, 0);
             drained = c >= n_in;
         }
+        if (drained && P.item_budget) {
+            const unsigned busy = __ballot_sync(kFull, s.active);
+            if (busy && busy != kFull) {
+                s = share_in_warp<SM, NW, T>(P, s, stk);
+                alive |= s.active;
+            }
+        }
         if (!__any_sync(kFull, alive)) break;
 
         // ---- steps: a warp-uniform trip count; a lane without work has an empty set at its
@@ -607,7 +682,7 @@ __global__ void __launch_bounds__(T, (NW == 1 && SM ? 768 : 512) / T) dfs_compac
                 s.entries = r.entries;
 #pragma unroll
                 for (int w = 0; w < NW; ++w) s.R[w] = r.m[w] & s.A[w];
-                fix = flagged<NW>(r, s.R);
+                fix = flagged<NW>(r);
                 above_slot<NW>(s.R, slot, bits.above);
                 popped = slot + 1;
             }
@@ -646,7 +721,7 @@ __global__ void __launch_bounds__(T, (NW == 1 && SM ? 768 : 512) / T) dfs_compac
                 solved = s.L == s.n - 1;  // level n has no candidate
                 // (3) down, when the next level has one
                 if (any<NW>(c)) {
-                    fix = flagged<NW>(r, c);
+                    fix = flagged<NW>(r);
 #pragma unroll
                     for (int w = 0; w < NW; ++w) {
                         const uint64_t o = s.O[w];
@@ -673,19 +748,18 @@ __global__ void __launch_bounds__(T, (NW == 1 && SM ? 768 : 512) / T) dfs_compac
             account<NW>(P, s);
             idle<NW>(s);
         }
+        if (drained && alone < 0x80000000u) alone += kStepsPerFetch;
         if (!s.active) continue;
-        s.steps += kStepsPerFetch;
         since_check += kStepsPerFetch;
 
         // ---- once the queue is empty, hand work back for the next round ----
-        if (drained && P.item_budget && s.steps >= P.item_budget) {
+        if (P.item_budget && alone >= P.item_budget) {
             if (split_state<SM, NW, T>(P, out, s, stk)) {
                 account<NW>(P, s);
                 idle<NW>(s);
                 alive = false;
                 continue;
             }
-            s.steps = 0;
         }
         // ---- deadline, cancellation and stop-at-first, every 4096 steps ----
         if (since_check >= 4096) {

@@ -218,7 +218,7 @@ std::vector<uint32_t> build_compact(const PuzzleModel& m, const std::vector<Leve
             for (size_t a = i; a < e; ++a) {
                 const Cand& q = k.cands[in[a].cand];
                 mask[static_cast<size_t>(r) * nw + (in[a].slot >> 6)] |= uint64_t(1) << (in[a].slot & 63u);
-                entries[info[r] + in[a].slot] = static_cast<uint16_t>(q.east << 4 | q.south << 9 | (q.t & 3u) << 14);
+                entries[info[r] + in[a].slot] = static_cast<uint16_t>((q.t & 3u) | q.east << 4 | q.south << 9);
                 for (size_t b = a + 1; b < e && !flag; ++b) {
                     const Cand& q2 = k.cands[in[b].cand];
                     flag = removes(k, q, q2) &&

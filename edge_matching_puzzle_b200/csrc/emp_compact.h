@@ -35,8 +35,8 @@
 //                      the slot in that word
 //   rows               row_bytes(NW) each, row 0 empty: NW candidate words (with the flag), byte
 //                      offset of slot 0 in the entries, word offset of the row's clears
-//   entries            16 bits per slot of a row: east colour << 4 | south colour << 9 |
-//                      orientation << 14 (only the slots of the row itself are there)
+//   entries            16 bits per slot of a row: orientation | east colour << 4 | south colour << 9
+//                      (only the slots of the row itself are there)
 //   -- the words up to here (hot) may be staged in shared memory --
 //   init[1 + NW]       availability of the border space and of the centre space (64 bits)
 //                      without the later twins

@@ -163,7 +163,7 @@ int main()
                 else C[slot >> 6] ^= k.toggle(space, slot);
                 std::vector<uint64_t> c = candidates(k, crow, cspace, C, B);
                 if (any(c)) {
-                    s.stk.at(L) = ((e >> 9) & 31u) | slot << 8 | static_cast<uint32_t>(any(R)) << 16 | space << 17 | row << 14;
+                    s.stk.at(L) = (e >> 9) | slot << 8 | static_cast<uint32_t>(any(R)) << 16 | space << 17 | row << 14;
                     s.C = C;
                     s.B = B;
                     ++L;
