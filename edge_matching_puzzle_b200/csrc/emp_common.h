@@ -26,7 +26,7 @@ emp_status select_device(int device, int* ordinal);
 // a pair on a B200 and a one-shot count makes some thirty: a 5x5 count took 6.5 ms, 0.04 ms of
 // it on the device.  Like cudaFree, device_free waits for the device, so no stream still uses what
 // goes back.  Safe from several threads; a device reset in between is noticed.
-constexpr uint64_t kPoolKeep = 1ull << 30, kPoolBlock = 256ull << 20;
+constexpr uint64_t kPoolKeep = 2ull << 30, kPoolBlock = 512ull << 20;
 cudaError_t device_alloc(void** p, size_t bytes, int* device, uint64_t* context);
 void device_free(void* p, int device, uint64_t context);
 

@@ -27,8 +27,8 @@ def test_freed_memory_kept_is_bounded():
     for _ in range(3):
         for h in handles:
             native.bt_count(h)
-    # the pool keeps at most 1 GiB; half as much again for what the driver keeps beside it
-    assert before - torch.cuda.mem_get_info()[0] <= 1536 << 20
+    # the pool keeps at most 2 GiB; a quarter as much again for what the driver keeps beside it
+    assert before - torch.cuda.mem_get_info()[0] <= 2560 << 20
 
 
 def test_counts_from_several_threads():
