@@ -24,9 +24,9 @@
 // What bounds it: instruction issue (74 % of the slots in the main rounds on a B200, 24 warps
 // an SM, shared-memory latency behind them); 30 of 32 lanes have work at a step, 22 of them a
 // candidate.  Measured, 1/64 of the 8x8 tree of 4 border / 8 interior colours, seed 0
-// (2.77e9 placements): 62.9 ms with dfs_kernel (4.4e10 placements/s), 25.7 ms here (1.08e11/s).
-// The step with selects in place of its two divergent regions took 27.6 ms, with the sharing
-// inside a warp inlined 26.1 ms (registers).
+// (2.77e9 placements): 62.9 ms with dfs_kernel (4.4e10 placements/s), 24.2 ms here (1.15e11/s).
+// It is short of registers (80 for 24 warps an SM): spilling six of them cost 1.5 ms, and so did a
+// second pop in a step.  Selects in place of the step's two divergent regions: 10 % slower.
 #include "emp_bt.h"
 
 #include <cuda_runtime.h>
@@ -64,9 +64,10 @@ __device__ __forceinline__ uint64_t ldg64(const uint32_t* p)
 
 template <int NW>
 struct Search {
-    uint64_t orig, nodes, sols;
-    const uint32_t* tb;              // the puzzle's blob
-    uint32_t pz, n, L, base, space;
+    uint64_t orig, nodes;
+    const uint32_t* tb;              // the puzzle's blob, number and levels: read by plans of several
+    uint32_t pz, n;                  // puzzles alone (blob, puzzle and levels below)
+    uint32_t L, base, space;
     int row;                         // byte offset of level L's row
     int entries;                     // byte offset of its slot 0 entry
     uint64_t R[NW];                  // candidates left at level L
@@ -80,6 +81,24 @@ struct Row {
     int entries;
     uint32_t clears;
 };
+
+// With staged tables the plan has one puzzle: its blob comes first and the rest is in the launch
+// parameters, which keeps six registers out of the search.
+template <bool SM, int NW>
+__device__ __forceinline__ const uint32_t* blob(const BtLaunch& P, const Search<NW>& s)
+{
+    return SM ? P.ctables : s.tb;
+}
+template <bool SM, int NW>
+__device__ __forceinline__ uint32_t puzzle(const Search<NW>& s)
+{
+    return SM ? 0u : s.pz;
+}
+template <bool SM, int NW>
+__device__ __forceinline__ uint32_t levels(const BtLaunch& P, const Search<NW>& s)
+{
+    return SM ? P.chdr.n : s.n;
+}
 
 struct SlotBits {
     uint64_t toggle, above;
@@ -234,13 +253,13 @@ __device__ __forceinline__ void only_tried(const uint32_t* id, uint64_t* r)
 // the current level's candidates: its row AND the availability, without those that other trials
 // of a flagged row remove
 template <bool SM, int NW>
-__device__ __forceinline__ void level_candidates(Search<NW>& s)
+__device__ __forceinline__ void level_candidates(const BtLaunch& P, Search<NW>& s)
 {
     const Row<NW> r = Tab<SM, NW>::row(s, s.row);
     s.entries = r.entries;
 #pragma unroll
     for (int w = 0; w < NW; ++w) s.R[w] = r.m[w] & s.A[w];
-    if (static_cast<int64_t>(r.m[NW - 1]) < 0) only_tried<NW>(s.tb + r.clears, s.R);
+    if (static_cast<int64_t>(r.m[NW - 1]) < 0) only_tried<NW>(blob<SM>(P, s) + r.clears, s.R);
 }
 
 // whether a row's trials have to be replayed
@@ -265,10 +284,10 @@ __device__ __forceinline__ void above_slot(uint64_t* r, uint32_t slot, uint64_t 
 
 // transition (kind_index << 2 | orientation) of a stack word
 template <bool SM, int NW>
-__device__ __forceinline__ uint32_t word_transition(const Search<NW>& s, uint32_t word)
+__device__ __forceinline__ uint32_t word_transition(const BtLaunch& P, const Search<NW>& s, uint32_t word)
 {
     const uint32_t slot = word_slot(word), space = word_space(word);
-    const uint32_t* tb = s.tb;
+    const uint32_t* tb = blob<SM>(P, s);
     uint32_t ki = __ldg(reinterpret_cast<const uint8_t*>(tb + __ldg(tb + 9)) + space * 64 * NW + slot);
     const uint32_t nborder = __ldg(tb + 11);
     if (space && ki >= nborder) ki -= nborder;
@@ -293,7 +312,6 @@ __device__ __forceinline__ void start_search(Search<NW>& s, uint32_t len)
     s.L = len;
     s.base = len;
     s.nodes = 0;
-    s.sols = 0;
     s.active = true;
 }
 
@@ -349,7 +367,7 @@ __device__ __forceinline__ void load_item(const BtLaunch& P, Search<NW>& s, cons
     }
     to_space<NW>(s, desc_space(Tab<SM, NW>::desc(s, len)));
     if (len < h.z) s.row = word_row(stk[len * T]);
-    level_candidates<SM, NW>(s);
+    level_candidates<SM, NW>(P, s);
     // after the piece placed at the level, or from the first slot left at the state's own level
     const uint32_t from = len < h.z ? word_slot(stk[len * T]) + 1 : g.y;
     if (from) above_slot<NW>(s.R, from - 1, Tab<SM, NW>::slot(P, s, s.space, from - 1).above);
@@ -364,13 +382,14 @@ __device__ __forceinline__ void load_record(const BtLaunch& P, Search<NW>& s, co
     s.orig = static_cast<uint64_t>(rec[0]) | (static_cast<uint64_t>(rec[1]) << 32);
     const uint32_t len = rec[2] & 0xFFFFu, start = rec[2] >> 16;
     start_puzzle<SM, NW>(P, s, rec[3] & 0xFFFFu);
-    const uint32_t init = __ldg(s.tb + 8), nborder = __ldg(s.tb + 11);
-    const uint32_t width = SM ? P.chdr.width : __ldg(s.tb + 2);
-    const uint8_t* first = reinterpret_cast<const uint8_t*>(s.tb + __ldg(s.tb + 10));
+    const uint32_t* tb = blob<SM>(P, s);
+    const uint32_t init = __ldg(tb + 8), nborder = __ldg(tb + 11);
+    const uint32_t width = SM ? P.chdr.width : __ldg(tb + 2);
+    const uint8_t* first = reinterpret_cast<const uint8_t*>(tb + __ldg(tb + 10));
 #pragma unroll
     for (int w = 0; w < NW; ++w) {
-        s.A[w] = ldg64(s.tb + init + 2 + 2 * w);
-        s.O[w] = w ? 0ull : ldg64(s.tb + init);
+        s.A[w] = ldg64(tb + init + 2 + 2 * w);
+        s.O[w] = w ? 0ull : ldg64(tb + init);
     }
     uint32_t west = 0;
     for (uint32_t l = 0;; ++l) {
@@ -381,7 +400,7 @@ __device__ __forceinline__ void load_record(const BtLaunch& P, Search<NW>& s, co
         if (l == len) break;
         const uint32_t t = (rec[4 + (l >> 1)] >> (16 * (l & 1))) & 0xFFFFu;
         // corners follow the borders in space 1
-        const bool corner = l == 0 || l + 1 == width || l + width == s.n || l + 1 == s.n;
+        const bool corner = l == 0 || l + 1 == width || l + width == levels<SM>(P, s) || l + 1 == levels<SM>(P, s);
         uint32_t slot = __ldg(first + 256 * s.space + (t >> 2) + (corner ? nborder : 0u));
         const int entries = Tab<SM, NW>::row(s, s.row).entries;
         uint32_t e = Tab<SM, NW>::entry(s, entries, slot);
@@ -391,12 +410,12 @@ __device__ __forceinline__ void load_record(const BtLaunch& P, Search<NW>& s, co
         stk[l * T] = make_word(e, slot, false, s.space, s.row);
         west = e;
     }
-    level_candidates<SM, NW>(s);
+    level_candidates<SM, NW>(P, s);
     if (start) {
         // a resumed level: drop the candidates below transition `start`
         while (any<NW>(s.R)) {
             const uint32_t slot = first_slot<NW>(s.R);
-            if (word_transition<SM, NW>(s, make_word(0, slot, false, s.space, s.row)) >= start) break;
+            if (word_transition<SM, NW>(P, s, make_word(0, slot, false, s.space, s.row)) >= start) break;
 #pragma unroll
             for (int w = 0; w < NW; ++w)
                 if (w == static_cast<int>(slot >> 6)) s.R[w] &= s.R[w] - 1;
@@ -410,9 +429,9 @@ __device__ __forceinline__ void load_record(const BtLaunch& P, Search<NW>& s, co
 template <bool SM, int NW, int T>
 __device__ __forceinline__ void record_solution(const BtLaunch& P, const Search<NW>& s, const uint32_t* stk)
 {
-    FirstRecord* r = P.first_records + s.pz;
-    atomicMin(&P.first_item[s.pz], (unsigned long long)s.orig);
-    if (s.orig > *(volatile unsigned long long*)&P.first_item[s.pz]) return;
+    FirstRecord* r = P.first_records + puzzle<SM>(s);
+    atomicMin(&P.first_item[puzzle<SM>(s)], (unsigned long long)s.orig);
+    if (s.orig > *(volatile unsigned long long*)&P.first_item[puzzle<SM>(s)]) return;
     const uint64_t give_up = global_ns() + P.first_lock_wait_ns;
     while (atomicCAS(&r->lock, 0u, 1u) != 0u) {
         if (global_ns() > give_up) {
@@ -425,8 +444,8 @@ __device__ __forceinline__ void record_solution(const BtLaunch& P, const Search<
     __threadfence();
     bool better = !r->has;
     if (!better) {
-        for (uint32_t l = 0; l < s.n; ++l) {
-            const uint32_t mine = word_transition<SM, NW>(s, stk[l * T]), theirs = r->t[l];
+        for (uint32_t l = 0; l < levels<SM>(P, s); ++l) {
+            const uint32_t mine = word_transition<SM, NW>(P, s, stk[l * T]), theirs = r->t[l];
             if (mine != theirs) {
                 better = mine < theirs;
                 break;
@@ -434,8 +453,8 @@ __device__ __forceinline__ void record_solution(const BtLaunch& P, const Search<
         }
     }
     if (better) {
-        for (uint32_t l = 0; l < s.n; ++l)
-            r->t[l] = static_cast<uint16_t>(word_transition<SM, NW>(s, stk[l * T]));
+        for (uint32_t l = 0; l < levels<SM>(P, s); ++l)
+            r->t[l] = static_cast<uint16_t>(word_transition<SM, NW>(P, s, stk[l * T]));
         r->has = 1;
     }
     __threadfence();
@@ -447,6 +466,8 @@ template <bool SM, int NW, int T>
 __device__ __noinline__ void solution_found(const BtLaunch& P, const Search<NW> s, const uint32_t* stk,
                                             uint32_t placed)
 {
+    atomicAdd(&P.totals[2 * puzzle<SM>(s) + 1], 1ull);
+    if (P.item_nodes) atomicAdd(&P.item_sols[s.orig], 1ull);
     record_solution<SM, NW, T>(P, s, stk);
     if (P.sols) {
         const unsigned long long at = atomicAdd(P.sol_count, 1ull);
@@ -454,8 +475,8 @@ __device__ __noinline__ void solution_found(const BtLaunch& P, const Search<NW> 
             SolutionRecord* r = P.sols + at;
             r->orig = s.orig;
             r->local = s.nodes + placed;
-            for (uint32_t l = 0; l < s.n; ++l)
-                r->t[l] = static_cast<uint16_t>(word_transition<SM, NW>(s, stk[l * T]));
+            for (uint32_t l = 0; l < levels<SM>(P, s); ++l)
+                r->t[l] = static_cast<uint16_t>(word_transition<SM, NW>(P, s, stk[l * T]));
         }
     }
     if (P.stop_at_any) {
@@ -465,14 +486,12 @@ __device__ __noinline__ void solution_found(const BtLaunch& P, const Search<NW> 
     }
 }
 
-template <int NW>
+template <bool SM, int NW>
 __device__ __forceinline__ void account(const BtLaunch& P, const Search<NW>& s)
 {
-    if (s.nodes) atomicAdd(&P.totals[2 * s.pz], (unsigned long long)s.nodes);
-    if (s.sols) atomicAdd(&P.totals[2 * s.pz + 1], (unsigned long long)s.sols);
+    if (s.nodes) atomicAdd(&P.totals[2 * puzzle<SM>(s)], (unsigned long long)s.nodes);
     if (P.item_nodes) {
         if (s.nodes) atomicAdd(&P.item_nodes[s.orig], (unsigned long long)s.nodes);
-        if (s.sols) atomicAdd(&P.item_sols[s.orig], (unsigned long long)s.sols);
     }
 }
 
@@ -498,7 +517,7 @@ __device__ __noinline__ bool split_state(const BtLaunch& P, uint32_t* out, const
     if (here) items[k] = (me << 32) | s.L;
     uint32_t* st = out + me * P.crec_words;
     *reinterpret_cast<uint4*>(st) =
-        make_uint4(static_cast<uint32_t>(s.orig), static_cast<uint32_t>(s.orig >> 32), s.L, s.pz);
+        make_uint4(static_cast<uint32_t>(s.orig), static_cast<uint32_t>(s.orig >> 32), s.L, puzzle<SM>(s));
     const uint64_t border = s.space ? s.A[0] : s.O[0];
     *reinterpret_cast<uint4*>(st + 4) = make_uint4(static_cast<uint32_t>(s.row), here ? first_slot<NW>(s.R) : 0u,
                                                    static_cast<uint32_t>(border), static_cast<uint32_t>(border >> 32));
@@ -536,7 +555,7 @@ __device__ __noinline__ Search<NW> share_in_warp(const BtLaunch& P, Search<NW> s
     const bool donor = open != ~0u && __popc(donors & lt) < __popc(idle);
     const uint32_t from = thief ? __fns(donors, 0, __popc(idle & lt) + 1) : lane;
     const uint32_t level = __shfl_sync(kFull, open, from), top = __shfl_sync(kFull, s.L, from);
-    const uint32_t space = __shfl_sync(kFull, s.space, from), pz = __shfl_sync(kFull, s.pz, from);
+    const uint32_t space = __shfl_sync(kFull, s.space, from), pz = __shfl_sync(kFull, puzzle<SM>(s), from);
     const uint64_t orig = __shfl_sync(kFull, s.orig, from);
     uint64_t a[NW], o[NW];
 #pragma unroll
@@ -564,7 +583,7 @@ __device__ __noinline__ Search<NW> share_in_warp(const BtLaunch& P, Search<NW> s
         const uint32_t word = col[level * T], slot = word_slot(word);
         to_space<NW>(s, word_space(word));
         s.row = word_row(word);
-        level_candidates<SM, NW>(s);
+        level_candidates<SM, NW>(P, s);
         above_slot<NW>(s.R, slot, Tab<SM, NW>::slot(P, s, s.space, slot).above);
         start_search<NW>(s, level);
     }
@@ -641,7 +660,7 @@ __global__ void __launch_bounds__(T, (NW == 1 && SM ? 768 : 512) / T) dfs_compac
                         } else {
                             if (items) load_item<SM, NW, T>(P, s, rec, static_cast<uint32_t>(item), stk);
                             else load_record<SM, NW, T>(P, s, rec, stk);
-                            if (P.stop_at_first && s.orig > *(volatile unsigned long long*)&P.first_item[s.pz])
+                            if (P.stop_at_first && s.orig > *(volatile unsigned long long*)&P.first_item[puzzle<SM>(s)])
                                 idle<NW>(s);  // a lower subtree of this puzzle holds a solution
                         }
                     }
@@ -689,7 +708,7 @@ __global__ void __launch_bounds__(T, (NW == 1 && SM ? 768 : 512) / T) dfs_compac
             // the trials of flagged rows, of a level popped to or just entered
             if (__any_sync(kFull, fix)) {
                 if (fix) {
-                    level_candidates<SM, NW>(s);
+                    level_candidates<SM, NW>(P, s);
                     if (popped) above_slot<NW>(s.R, popped - 1, TB::slot(P, s, s.space, popped - 1).above);
                     fix = false;
                 }
@@ -718,7 +737,7 @@ __global__ void __launch_bounds__(T, (NW == 1 && SM ? 768 : 512) / T) dfs_compac
                     a[w] = s.A[w] ^ (NW == 1 || w == static_cast<int>(slot >> 6) ? bits : 0ull);
                     c[w] = r.m[w] & (same ? a[w] : s.O[w]);
                 }
-                solved = s.L == s.n - 1;  // level n has no candidate
+                solved = s.L == levels<SM>(P, s) - 1;  // level n has no candidate
                 // (3) down, when the next level has one
                 if (any<NW>(c)) {
                     fix = flagged<NW>(r);
@@ -737,7 +756,6 @@ __global__ void __launch_bounds__(T, (NW == 1 && SM ? 768 : 512) / T) dfs_compac
             }
             if (__any_sync(kFull, solved)) {
                 if (solved) {
-                    ++s.sols;
                     solution_found<SM, NW, T>(P, s, stk, placed);
                 }
                 __syncwarp();
@@ -745,7 +763,7 @@ __global__ void __launch_bounds__(T, (NW == 1 && SM ? 768 : 512) / T) dfs_compac
         }
         s.nodes += placed;
         if (s.active && !any<NW>(s.R) && s.L == s.base) {
-            account<NW>(P, s);
+            account<SM, NW>(P, s);
             idle<NW>(s);
         }
         if (drained && alone < 0x80000000u) alone += kStepsPerFetch;
@@ -755,7 +773,7 @@ __global__ void __launch_bounds__(T, (NW == 1 && SM ? 768 : 512) / T) dfs_compac
         // ---- once the queue is empty, hand work back for the next round ----
         if (P.item_budget && alone >= P.item_budget) {
             if (split_state<SM, NW, T>(P, out, s, stk)) {
-                account<NW>(P, s);
+                account<SM, NW>(P, s);
                 idle<NW>(s);
                 alive = false;
                 continue;
@@ -770,13 +788,13 @@ __global__ void __launch_bounds__(T, (NW == 1 && SM ? 768 : 512) / T) dfs_compac
                 atomicOr(P.status, EMP_DEV_TIMEOUT);
             }
             const bool superseded =
-                P.stop_at_first && s.orig > *(volatile unsigned long long*)&P.first_item[s.pz];
+                P.stop_at_first && s.orig > *(volatile unsigned long long*)&P.first_item[puzzle<SM>(s)];
             if (superseded || stop) {
-                account<NW>(P, s);
+                account<SM, NW>(P, s);
                 if (stop) {
                     // the lane stays alive: it goes on taking records only to mark
                     // their puzzles incomplete, so every dropped piece of work is known
-                    P.incomplete[s.pz] = 1u;
+                    P.incomplete[puzzle<SM>(s)] = 1u;
                     atomicExch(P.abort_flag, 1);
                     atomicOr(P.status, EMP_DEV_ABORTED);
                 } else {
