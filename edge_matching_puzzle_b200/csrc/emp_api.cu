@@ -536,7 +536,15 @@ emp_status create_plan(const emp_puzzle* puzzles, uint32_t count, const emp_bt_c
         }
         return EMP_OK;
     };
+    // the compact search with staged tables is built for 128-thread blocks (emp_btc.cu) while they
+    // give it 16 warps an SM
+    const bool small_blocks = pl->compact && pl->smem_tab_words && !pl->cfg.threads_per_block;
+    if (small_blocks) candidates = {128};
     EMP_TRY(pick_geometry());
+    if (small_blocks && best_warps < 16) {
+        candidates = {128, 256, 512};
+        EMP_TRY(pick_geometry());
+    }
     if (default_stack && pl->stack_mode == emp::kStackShared32 && best_warps < (pl->compact && count > 1 ? 8 : 16)) {
         pl->stack_mode = emp::kStackGlobal32;
         EMP_TRY(pick_geometry());

@@ -24,9 +24,11 @@
 // What bounds it: instruction issue (74 % of the slots in the main rounds on a B200, 24 warps
 // an SM, shared-memory latency behind them); 30 of 32 lanes have work at a step, 22 of them a
 // candidate.  Measured, 1/64 of the 8x8 tree of 4 border / 8 interior colours, seed 0
-// (2.77e9 placements): 62.9 ms with dfs_kernel (4.4e10 placements/s), 24.2 ms here (1.15e11/s).
-// It is short of registers (80 for 24 warps an SM): spilling six of them cost 1.5 ms, and so did a
-// second pop in a step.  Selects in place of the step's two divergent regions: 10 % slower.
+// (2.77e9 placements): 62.9 ms with dfs_kernel (4.4e10 placements/s), 23.4 ms here (1.18e11/s).
+// 128-thread blocks, five an SM, leave a thread 96 registers: 20 warps at 23.4 ms, where 24 warps
+// of 80 registers (256-thread blocks) take 24.2 ms and 16 of 128 registers 24.0 ms; on
+// 1/1024 of the tree 3.07 against 3.4 ms.  Tried and slower: selects in place of the step's two
+// divergent regions (10 %), a second pop in a step (5 %).
 #include "emp_bt.h"
 
 #include <cuda_runtime.h>
@@ -600,7 +602,7 @@ __device__ __noinline__ Search<NW> share_in_warp(const BtLaunch& P, Search<NW> s
 // cancellation and stop-at-first flags are those of dfs_kernel.  Work goes back to the queue for
 // the next round once a warp has searched on for the split budget after the queue ran empty.
 template <int NW, bool SM, bool GS, int T, int kStepsPerFetch>
-__global__ void __launch_bounds__(T, (NW == 1 && SM ? 768 : 512) / T) dfs_compact_kernel(const __grid_constant__ BtLaunch P)
+__global__ void __launch_bounds__(T, (NW == 1 && SM ? (T == 128 ? 640 : 768) : 512) / T) dfs_compact_kernel(const __grid_constant__ BtLaunch P)
 {
     using TB = Tab<SM, NW>;
     const uint32_t tid = threadIdx.x, lane = tid & 31;
@@ -806,7 +808,10 @@ __global__ void __launch_bounds__(T, (NW == 1 && SM ? 768 : 512) / T) dfs_compac
     }
 }
 
-constexpr int kSteps = 32;
+// steps between looks at the queue: 16, 32 and 64 took 24.7, 24.2 and 25.1 ms on 1/64 of the
+// seed-0 8x8 tree in 256-thread blocks; 32 and 48 took 23.3 and 23.5 ms in 128-thread blocks,
+// and 3.17 and 3.07 ms on 1/1024 of it
+constexpr int kSteps = 48;
 
 template <int NW, int T>
 const void* symbol_t(bool sm, bool gs)
