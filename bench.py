@@ -52,9 +52,9 @@ UNIT = "placements/s"
 WORKLOAD = (f"exhaustive row-major count of 16 seeded {WIDTH}x{HEIGHT} puzzles ({BORDER} border / {INTERIOR} interior "
             f"colours, seeds 0..15), split depth {DEPTH}, one step = 1/{SLICES} slice of the depth-{DEPTH} subtrees")
 L2_BYTES = 126 * 1024 * 1024
-# DRAM bytes (read + write) of one dfs_kernel round on this workload, from one ncu capture
-# (dfs_kernel<3, shared tables, 256 threads, shared 32-bit stack>, round 4 of the seed-0 slice)
-DFS_LAUNCH_DRAM_BYTES = 181.3e6
+# DRAM bytes (read + write) of one dfs_compact_kernel round on this workload, from one ncu capture
+# (one word, shared tables, shared stack, 128 threads, round 4 of the seed-0 slice)
+DFS_LAUNCH_DRAM_BYTES = 41.6e6
 
 
 def env_int(name, default):
@@ -131,14 +131,15 @@ def make_puzzles():
     return [native.NativePuzzle(WIDTH, HEIGHT, native.generate(WIDTH, HEIGHT, BORDER, INTERIOR, s)) for s in SEEDS]
 
 
-def algorithmic_work(kind_nodes, puzzle):
-    """Per-placement work of the search (32-bit words W_k of the placed kind's
-    bitfield): I = 4*W_k + 8 integer ops, S = 16*W_k bytes of table/state traffic
-    (read table row, read availability, write availability, write the remaining
-    candidate set).  Weighted by the node mix per kind."""
+def algorithmic_work(kind_nodes, puzzle, bitfield=False):
+    """Per-placement work of the search (32-bit words W_k of a level's candidate set):
+    I = 4*W_k + 8 integer ops, S = 16*W_k bytes of table/state traffic (read table row,
+    read availability, write availability, write the remaining candidate set).  Weighted
+    by the node mix per kind.  The row-major search holds a candidate set in one 64-bit
+    word; the bitfield search (an explicit stack placement) has 4 bits per piece."""
     info = puzzle.info()
     nk = [info.nb_center, info.nb_border, info.nb_corner]
-    wk = [(4 * n + 31) // 32 for n in nk]
+    wk = [(4 * n + 31) // 32 for n in nk] if bitfield else [2, 2, 2]
     total = sum(kind_nodes) or 1
     ops = sum((4 * wk[k] + 8) * kind_nodes[k] for k in range(3)) / total
     byts = sum(16 * wk[k] * kind_nodes[k] for k in range(3)) / total
@@ -794,6 +795,7 @@ def main():
     busy = 0.0
     rounds = 0
     records = 0
+    bitfield = args.stack_placement != 0
     launches = 0
     step_ms = []
     dev_index = torch.cuda.current_device()
@@ -814,10 +816,15 @@ def main():
             nodes += sum(r.nodes for r in res)
             busy += sum(r.dfs_busy_ms for r in res)
             rounds += sum(r.rounds for r in res)
-            records += sum(r.work_records + r.handed_back for r in res)
-            if graphs:  # make_records, reset; per round a DFS launch, the round controller and (after the
-                # first) the record copy
-                launches += sum(2 + 3 * r.rounds - 1 for r in res)
+            moved = sum(r.work_records + r.handed_back for r in res)
+            if bitfield:
+                records += 4 * plans[0].rec_words() * moved
+            else:  # an initial record is a header and the prefix, a handed-back item 8 bytes (written and read)
+                first = sum(pl.selected for pl in plans)
+                records += 4 * (4 + DEPTH // 2) * first + 8 * (moved - first)
+            if graphs:  # make_records, reset; per round a DFS launch, the round controller and (bitfield
+                # search, after the first) the record copy
+                launches += sum(2 + (3 * r.rounds - 1 if bitfield else 2 * r.rounds) for r in res)
             else:  # make_records + reset + one DFS launch per round
                 launches += sum(2 + r.rounds for r in res)
     sampler.__exit__()
@@ -881,15 +888,14 @@ def main():
     if rank == 0:
         if kinds is None:
             kinds = [85, 14, 1]
-        ops, byts, mix = algorithmic_work(kinds, puzzles[0])
+        ops, byts, mix = algorithmic_work(kinds, puzzles[0], bitfield)
         # host-loop runs time every DFS launch with events; graph runs (puzzles on concurrent
         # streams, rounds launched by the device) give the timed region per launch, which
-        # also holds the small record-copy and round-controller kernels
+        # also holds the small round-controller kernels
         launch_ms = (busy if not graphs else ms) / max(rounds, 1)
         placements_per_launch = nodes / max(rounds, 1)
         sm_clock = (clocks or {}).get("sm_max_mhz") or peaks.get("sm_max_mhz", 1965.0)
-        rec_bytes = 4 * plans[0].rec_words()
-        dram_alg = records * rec_bytes / max(rounds, 1)  # work records read and written per launch
+        dram_alg = records / max(rounds, 1)  # bytes of work records and items read and written per launch
         out = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms_max / args.steps, "higher_is_better": True,
@@ -902,13 +908,13 @@ def main():
                          "peak": peaks["hbm_gbs"], "unit": "GB/s",
                          "frac": dram_alg / (launch_ms / 1000) / 1e9 / peaks["hbm_gbs"],
                          "traffic": DFS_LAUNCH_DRAM_BYTES,
-                         "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one dfs_kernel round "
+                         "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one dfs_compact_kernel round "
                                            "(seed-0 slice, same grid and table staging; caches flushed by ncu)",
                          "peak_source": peak_kind,
-                         "note": "dfs_kernel keeps its state on chip; DRAM only carries work records, so the "
+                         "note": "the search keeps its state on chip; DRAM only carries work records, so the "
                                  "on-chip roofline below is the binding one"},
             "roofline_onchip": {
-                "kernel": "dfs_kernel", "launch_ms": launch_ms, "placements_per_launch": placements_per_launch,
+                "kernel": "dfs_kernel" if bitfield else "dfs_compact_kernel", "launch_ms": launch_ms, "placements_per_launch": placements_per_launch,
                 "int_ops_per_placement": ops, "smem_bytes_per_placement": byts, "node_mix_center_border_corner": mix,
                 # integer instructions issue on the ALU pipe (logic, shifts, compares: ncu's
                 # sm__inst_executed_pipe_alu.avg.peak_sustained = 2 warp instructions per SM

@@ -21,11 +21,11 @@
 // (more: candidates remained after this one was taken).  A is the availability of the space
 // of the current level and O the other one; they change places when the level's space does.
 //
-// What bounds it: instruction issue (74 % of the slots in the main rounds on a B200, 24 warps
-// an SM, shared-memory latency behind them); 30 of 32 lanes have work at a step, 22 of them a
-// candidate.  Measured, 1/64 of the 8x8 tree of 4 border / 8 interior colours, seed 0
-// (2.77e9 placements): 62.9 ms with dfs_kernel (4.4e10 placements/s), 23.4 ms here (1.18e11/s).
-// 128-thread blocks, five an SM, leave a thread 96 registers: 20 warps at 23.4 ms, where 24 warps
+// What bounds it: integer instructions (ALU pipe 78.5 % and issue slots 76.8 % busy in the main
+// rounds on a B200, 21 lanes in an instruction, 20 warps an SM, which hide the shared-memory
+// latency); 30 of 32 lanes have work at a step, 22 of them a candidate.  Measured, 1/64 of the
+// 8x8 tree of 4 border / 8 interior colours, seed 0 (2.77e9 placements): 62.9 ms with dfs_kernel (4.4e10 placements/s), 23.4 ms here (1.18e11/s).
+// 128-thread blocks, five an SM, let a thread have its 90 registers: 20 warps at 23.4 ms, where 24 warps
 // of 80 registers (256-thread blocks) take 24.2 ms and 16 of 128 registers 24.0 ms; on
 // 1/1024 of the tree 3.07 against 3.4 ms.  Tried and slower: selects in place of the step's two
 // divergent regions (10 %), a second pop in a step (5 %).

@@ -526,7 +526,7 @@ class BtPlan:
         return list(buf)
 
     def rec_words(self) -> int:
-        """32-bit words per work record (header, prefix, remaining set)."""
+        """32-bit words per work record of the bitfield search (header, prefix, remaining set)."""
         n = max(p.n for p in self.puzzles)
         kw = max(p.max_kind_words() for p in self.puzzles)
         return 4 + (n + 1) // 2 + 2 * kw

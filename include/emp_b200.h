@@ -101,7 +101,8 @@ emp_status emp_puzzle_export_tables(emp_puzzle puzzle, uint32_t *out, uint64_t c
 
 typedef struct emp_bt_config {
     uint32_t split_depth;        /* levels expanded before subtrees go to threads; 0 = auto */
-    uint32_t threads_per_block;  /* 128, 256 or 512; 0 = the size with the most resident warps */
+    uint32_t threads_per_block;  /* 128, 256 or 512; 0 = 128 in the row-major search of one puzzle,
+                                    else the size with the most resident warps */
     uint32_t blocks_per_sm;      /* 0 = as many as fit */
     uint32_t stop_at_first;      /* 1: stop once the reference's first solution is known */
     uint64_t reserved_budget;    /* unused, keep 0 */
@@ -131,9 +132,10 @@ typedef struct emp_bt_config {
                                     A wait that runs out reports EMP_FIRST_LOST for the puzzle */
     uint32_t hold_first_lock;    /* testing only: 1 = every first-solution record starts locked by
                                     nobody, so each wait runs out (exercises EMP_FIRST_LOST) */
-    uint32_t stack_placement;    /* where each thread keeps its DFS stack: 0 = default (1 when
-                                    the tables are staged in shared memory and 1 leaves at
-                                    least 16 warps per SM, else 3),
+    uint32_t stack_placement;    /* where each thread keeps its DFS stack: 0 = default (the
+                                    row-major search where it applies, else the bitfield search
+                                    with 1 when the tables are staged in shared memory and 1
+                                    leaves at least 16 warps per SM, else 3); bitfield search:
                                     1 = shared memory, 32-bit entries with the placed piece's colours,
                                     2 = shared memory, 16-bit entries (more threads per SM; colours are
                                         read from the transition table),
