@@ -704,6 +704,84 @@ emp_status build_graph(emp_bt_plan_t& pl)
 
 }  // namespace
 
+namespace {
+
+// A run whose rounds the host launches: the initial records, then the work handed back by each
+// round.  A round is in flight between start() or finish_round() and the next finish_round().
+class RoundLoop {
+public:
+    RoundLoop(emp_bt_plan_t& plan, cudaStream_t stream) : pl_(plan), st_(stream) {}
+    bool active() const { return n_in_ != 0; }
+
+    emp_status start()
+    {
+        pl_.graph_ran = false;
+        P_ = pl_.launch();
+        CUDA_TRY(emp::launch_bt_reset(P_, static_cast<uint32_t>(pl_.puzzles.size()), st_));
+        if (pl_.item_nodes.p) {
+            CUDA_TRY(cudaMemsetAsync(pl_.item_nodes.p, 0, pl_.item_nodes.bytes, st_));
+            CUDA_TRY(cudaMemsetAsync(pl_.item_sols.p, 0, pl_.item_sols.bytes, st_));
+        }
+        CUDA_TRY(cudaEventRecord(pl_.ev0, st_));
+        in_ = pl_.rec_init.as<uint32_t>();
+        n_in_ = pl_.n_init;
+        out_ = &pl_.rec_a;
+        spare_ = &pl_.rec_b;
+        pl_.rounds = 0;
+        pl_.busy_ms = 0;
+        pl_.records_in = 0;
+        pl_.records_out = 0;
+        return launch();
+    }
+
+    emp_status finish_round()
+    {
+        unsigned long long tail = 0;
+        CUDA_TRY(cudaMemcpyAsync(&tail, pl_.counters.as<unsigned long long>() + 1, sizeof(tail),
+                                 cudaMemcpyDeviceToHost, st_));
+        CUDA_TRY(cudaStreamSynchronize(st_));
+        float rms = 0;
+        CUDA_TRY(cudaEventElapsedTime(&rms, pl_.evr0, pl_.evr1));
+        pl_.busy_ms += rms;
+        n_in_ = std::min<uint64_t>(tail, pl_.capacity);
+        pl_.records_out += n_in_;
+        in_ = out_->as<uint32_t>();
+        std::swap(out_, spare_);
+        if (pl_.rounds > kMaxRounds) return fail(EMP_ERR_CUDA, "emp_bt_plan_run: too many rounds");
+        return launch();
+    }
+
+private:
+    emp_status launch()  // the next round, or the end of the run
+    {
+        if (!n_in_) {
+            CUDA_TRY(cudaEventRecord(pl_.ev1, st_));
+            pl_.ran = true;
+            return EMP_OK;
+        }
+        pl_.records_in += n_in_;
+        CUDA_TRY(cudaMemsetAsync(pl_.counters.p, 0, pl_.counters.bytes, st_));
+        P_.in_rec = in_;
+        P_.n_in = n_in_;
+        P_.out_rec = out_->as<uint32_t>();
+        CUDA_TRY(cudaEventRecord(pl_.evr0, st_));
+        P_.in_items = pl_.rounds != 0;
+        CUDA_TRY(pl_.launch_round(P_, st_));
+        CUDA_TRY(cudaEventRecord(pl_.evr1, st_));
+        ++pl_.rounds;
+        return EMP_OK;
+    }
+
+    emp_bt_plan_t& pl_;
+    cudaStream_t st_;
+    emp::BtLaunch P_{};
+    const uint32_t* in_ = nullptr;
+    uint64_t n_in_ = 0;
+    DeviceBuffer *out_ = nullptr, *spare_ = nullptr;
+};
+
+}  // namespace
+
 extern "C" emp_status emp_bt_plan_run(emp_bt_plan plan, void* stream)
 {
     emp::clear_error();
@@ -726,49 +804,9 @@ extern "C" emp_status emp_bt_plan_run(emp_bt_plan plan, void* stream)
         plan->ran = true;
         return EMP_OK;
     }
-    plan->graph_ran = false;
-    emp::BtLaunch P = plan->launch();
-    CUDA_TRY(emp::launch_bt_reset(P, static_cast<uint32_t>(plan->puzzles.size()), st));
-    if (plan->item_nodes.p) {
-        CUDA_TRY(cudaMemsetAsync(plan->item_nodes.p, 0, plan->item_nodes.bytes, st));
-        CUDA_TRY(cudaMemsetAsync(plan->item_sols.p, 0, plan->item_sols.bytes, st));
-    }
-    CUDA_TRY(cudaEventRecord(plan->ev0, st));
-    // rounds: the initial records, then the work handed back by each round
-    const uint32_t* in = plan->rec_init.as<uint32_t>();
-    uint64_t n_in = plan->n_init;
-    DeviceBuffer* out = &plan->rec_a;
-    DeviceBuffer* spare = &plan->rec_b;
-    plan->rounds = 0;
-    plan->busy_ms = 0;
-    plan->records_in = 0;
-    plan->records_out = 0;
-    while (n_in) {
-        plan->records_in += n_in;
-        CUDA_TRY(cudaMemsetAsync(plan->counters.p, 0, plan->counters.bytes, st));
-        P.in_rec = in;
-        P.n_in = n_in;
-        P.out_rec = out->as<uint32_t>();
-        CUDA_TRY(cudaEventRecord(plan->evr0, st));
-        P.in_items = plan->rounds != 0;
-        CUDA_TRY(plan->launch_round(P, st));
-        CUDA_TRY(cudaEventRecord(plan->evr1, st));
-        ++plan->rounds;
-        unsigned long long tail = 0;
-        CUDA_TRY(cudaMemcpyAsync(&tail, plan->counters.as<unsigned long long>() + 1, sizeof(tail),
-                                 cudaMemcpyDeviceToHost, st));
-        CUDA_TRY(cudaStreamSynchronize(st));
-        float rms = 0;
-        CUDA_TRY(cudaEventElapsedTime(&rms, plan->evr0, plan->evr1));
-        plan->busy_ms += rms;
-        n_in = std::min<uint64_t>(tail, plan->capacity);
-        plan->records_out += n_in;
-        in = out->as<uint32_t>();
-        std::swap(out, spare);
-        if (plan->rounds > kMaxRounds) return fail(EMP_ERR_CUDA, "emp_bt_plan_run: too many rounds");
-    }
-    CUDA_TRY(cudaEventRecord(plan->ev1, st));
-    plan->ran = true;
+    RoundLoop loop(*plan, st);
+    EMP_TRY(loop.start());
+    while (loop.active()) EMP_TRY(loop.finish_round());
     return EMP_OK;
 }
 
@@ -871,22 +909,79 @@ extern "C" void emp_bt_plan_destroy(emp_bt_plan plan)
 
 namespace {
 
+emp_status sampled_plan(const emp_puzzle* puzzles, uint32_t count, const emp_bt_config* config,
+                        std::unique_ptr<emp_bt_plan_t>& out)
+{
+    emp_bt_plan plan = nullptr;
+    const emp_status s = emp_bt_plan_create(puzzles, count, config, &plan);
+    if (s != EMP_OK) return s;
+    out.reset(plan);
+    if (!config || !config->sample_stride) return EMP_OK;
+    const uint64_t first = config->sample_first, stride = config->sample_stride;
+    const uint64_t n = first < plan->n_all ? (plan->n_all - first + stride - 1) / stride : 0;
+    return emp_bt_plan_select(plan, first, stride, n);
+}
+
 emp_status count_one_plan(const emp_puzzle* puzzles, uint32_t count, const emp_bt_config* config,
                           emp_bt_result* results)
 {
-    emp_bt_plan plan = nullptr;
-    emp_status s = emp_bt_plan_create(puzzles, count, config, &plan);
-    if (s != EMP_OK) return s;
-    std::unique_ptr<emp_bt_plan_t> guard(plan);
-    if (config && config->sample_stride) {
-        const uint64_t first = config->sample_first, stride = config->sample_stride;
-        const uint64_t n = first < plan->n_all ? (plan->n_all - first + stride - 1) / stride : 0;
-        s = emp_bt_plan_select(plan, first, stride, n);
-        if (s != EMP_OK) return s;
+    std::unique_ptr<emp_bt_plan_t> plan;
+    EMP_TRY(sampled_plan(puzzles, count, config, plan));
+    EMP_TRY(emp_bt_plan_run(plan.get(), nullptr));
+    return emp_bt_plan_results(plan.get(), results);
+}
+
+// Puzzles with a plan each, run up to four at a time on their plans' own streams: a search's last,
+// small rounds leave most of the chip idle, and another search's rounds fill it.  No more plans are
+// added once they hold 512 MiB (an 8x8 board's holds about 120 MB), so that the memory of later
+// groups comes from the pool.  A plan that cannot be made beside others is made again alone.
+// Measured on a B200, 1/64 of four 8x8 trees (2.95e9 placements), a whole call:
+// 37.6 ms one after the other, 31.6 ms side by side.
+emp_status count_side_by_side(const emp_puzzle* puzzles, uint32_t count, const emp_bt_config* config,
+                              emp_bt_result* results)
+{
+    constexpr uint32_t kSide = 4;
+    constexpr uint64_t kSideBytes = 512ull << 20;
+    bool alone = false;
+    for (uint32_t done = 0; done < count;) {
+        std::vector<std::unique_ptr<emp_bt_plan_t>> plans;
+        uint64_t held = 0;
+        emp_status s = EMP_OK;
+        while (done + plans.size() < count && plans.size() < (alone ? 1u : kSide) && held < kSideBytes) {
+            std::unique_ptr<emp_bt_plan_t> pl;
+            s = sampled_plan(&puzzles[done + plans.size()], 1, config, pl);
+            if (s != EMP_OK) break;
+            held += pl->prefixes.bytes + pl->rec_init.bytes + pl->rec_a.bytes + pl->rec_b.bytes + pl->stack.bytes +
+                    pl->spill.bytes;
+            plans.push_back(std::move(pl));
+        }
+        if (s != EMP_OK && plans.empty()) return s;
+        alone = s != EMP_OK;
+        if (alone) cudaGetLastError();  // a refused allocation is not an error of the next launch
+        CUDA_TRY(cudaStreamSynchronize(nullptr));  // the plans' streams do not wait for the one that filled them
+        std::vector<RoundLoop> loops;
+        for (auto& pl : plans) loops.emplace_back(*pl, pl->select_stream);
+        // a failed step still waits for the others' rounds before the plans go
+        s = EMP_OK;
+        auto step = [&s](emp_status r) { if (s == EMP_OK) s = r; };
+        for (auto& l : loops)
+            if (s == EMP_OK) step(l.start());
+        for (bool any = true; any && s == EMP_OK;) {
+            any = false;
+            for (auto& l : loops)
+                if (s == EMP_OK && l.active()) {
+                    step(l.finish_round());
+                    any = true;
+                }
+        }
+        if (s != EMP_OK) {
+            for (auto& pl : plans) cudaStreamSynchronize(pl->select_stream);
+            return s;
+        }
+        for (auto& pl : plans) EMP_TRY(emp_bt_plan_results(pl.get(), &results[done++]));
     }
-    s = emp_bt_plan_run(plan, nullptr);
-    if (s != EMP_OK) return s;
-    return emp_bt_plan_results(plan, results);
+    emp::clear_error();  // of a plan that did not fit beside the others
+    return EMP_OK;
 }
 
 }  // namespace
@@ -903,7 +998,13 @@ extern "C" emp_status emp_bt_count_batch(const emp_puzzle* puzzles, uint32_t cou
     for (uint32_t i = 0; i < count && separate; ++i) separate = puzzles[i] && puzzles[i]->model.n >= 36;
     emp_status s = EMP_OK;
     if (separate && count > 1) {
-        for (uint32_t i = 0; i < count && s == EMP_OK; ++i) s = count_one_plan(&puzzles[i], 1, config, &results[i]);
+        // under a deadline, with an early stop or as graphs: one after the other
+        if (config && (config->timeout_ms || config->stop_at_first || config->stop_at_any || config->use_graph)) {
+            for (uint32_t i = 0; i < count && s == EMP_OK; ++i)
+                s = count_one_plan(&puzzles[i], 1, config, &results[i]);
+        } else {
+            s = count_side_by_side(puzzles, count, config, results);
+        }
     } else {
         s = count_one_plan(puzzles, count, config, results);
     }

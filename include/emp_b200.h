@@ -156,7 +156,8 @@ typedef struct emp_bt_result {
     uint32_t split_depth;        /* this puzzle's split depth */
     uint32_t has_first_solution;
     uint32_t first_solution[256];/* per board position y*w+x: (piece id-1)<<2 | orientation */
-    double kernel_ms;            /* DFS kernel time (device events, all rounds) */
+    double kernel_ms;            /* DFS kernel time (device events, all rounds); the searches of one
+                                    emp_bt_count_batch call may run side by side, and their times overlap */
     double total_ms;             /* whole call, host clock */
     uint32_t rounds;             /* DFS rounds (work handed back between rounds) */
     uint32_t first_found_us;     /* device time from the start of the run to the first solution

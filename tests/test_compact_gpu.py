@@ -10,7 +10,7 @@ import functools
 import pytest
 
 from edge_matching_puzzle_b200 import native
-from edge_matching_puzzle_b200.puzzle import generate
+from edge_matching_puzzle_b200.puzzle import generate, spiral_order
 from oracle.oracle import OraclePuzzle
 
 pytestmark = pytest.mark.gpu
@@ -68,3 +68,22 @@ def test_four_words_sampled_subtrees(kw):
     nodes, sols = plan.subtree_counts(sample)
     assert list(zip(nodes, sols)) == want
     assert (res.nodes, res.solutions) == (sum(nodes), sum(sols))
+
+
+@pytest.mark.parametrize("count", [2, 4, 5, 11])
+@pytest.mark.parametrize("kw", [{}, {"keep_subtree_counts": 1, "split_budget": 1}, {"stack_placement": 1},
+                                {"timeout_ms": 60000}], ids=str)
+def test_puzzles_side_by_side_equal_oracle(count, kw):
+    """A call with a few bigger puzzles runs their searches side by side, in groups: wide boards, a
+    spiral order and trees of very different sizes in one call."""
+    shapes = [(8, 8, 5, 12, 0), (6, 6, 4, 8, 1), (9, 9, 8, 20, 1), (12, 9, 9, 21, 0), (6, 7, 4, 9, 2), (10, 10, 8, 21, 1),
+              (6, 6, 4, 7, 4), (8, 8, 5, 12, 1), (7, 7, 4, 9, 3), (6, 6, 4, 8, 5), (9, 9, 8, 20, 2)]
+    pzs = [generate(*b) for b in shapes[:count]]
+    orders = [spiral_order(p.width, p.height) if i % 5 == 1 else None for i, p in enumerate(pzs)]
+    want = [OraclePuzzle(p.width, p.height, p.colors).run(order=o)[0] for p, o in zip(pzs, orders)]
+    handles = [native.NativePuzzle(p.width, p.height, p.colors, order=o) for p, o in zip(pzs, orders)]
+    got = native.bt_count_batch(handles, split_depth=8, **kw)
+    assert [(r.status, r.nodes, r.solutions) for r in got] == [(native.EMP_OK, w.nodes, w.solutions) for w in want]
+    for p, r, w in zip(pzs, got, want):
+        if w.solutions:
+            assert list(r.first_solution)[: p.nb_pieces] == list(w.first_board)[: p.nb_pieces]
