@@ -642,6 +642,9 @@ __global__ void __launch_bounds__(T, (NW == 1 && SM ? (T == 128 ? 640 : 768) : 5
 
     for (;; ++iteration) {
         // ---- work fetch: one atomic per warp, ranks from the ballot ----
+        // a lane that dropped its work (handed back, stopped, superseded) may have just entered a
+        // flagged row: what it takes next starts from sets whose trials are replayed already
+        if (!s.active) fix = false;
         if (drained && !s.active) alive = false;
         const bool need = alive && !s.active;
         const unsigned needmask = __ballot_sync(kFull, need);
