@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(kInferThreads, 1)
 // layer 1 forward 96 us and bias 4 us -> 37 us (128 blocks of 8 warps: latency), its weight
 // gradient 179 us -> 21 us, a whole loss and gradient 0.95 ms -> 0.14 ms; the gradient's error
 // against 64 bits 4e-7 .. 1e-6 -> 8e-8, for the sums are shorter.
-constexpr int kTile = 64, kTk = 16, kTs = kTile + 4;
+constexpr int kTile = kMlpTile, kTk = 16, kTs = kTile + 4;
 
 enum class Epilogue {
     kBiasRelu,  // C = max(v + bias[n], 0)
@@ -618,7 +618,7 @@ __global__ void loss_kernel(const float* __restrict__ s, const float* __restrict
 
 // Rows of 32, a thread a column: d = ds / sum of weights; dh2 = d (x) w3 where h2 > 0, and the partial
 // sums of dw3 = h2^T d, db2 = column sums of dh2 and db3 = sum of d, [block][2 * kMlpHidden + 1].
-constexpr uint32_t kColRows = 32, kColParts = 2 * kMlpHidden + 1;
+constexpr uint32_t kColRows = kMlpColRows, kColParts = kMlpColParts;
 
 __global__ void __launch_bounds__(kMlpHidden)
     backward_columns_kernel(const float* __restrict__ ds, const float* __restrict__ h2, const float* __restrict__ params,
@@ -865,34 +865,11 @@ cudaError_t launch_mlp_infer_tc(const MlpDevice& m, const void* image, uint64_t 
     return cudaGetLastError();
 }
 
-namespace {
-
-// rows of a partial sum over `n` rows: at least 128 (a multiple of 16), at most `most` parts
-uint32_t part_rows(uint64_t n, uint32_t most)
-{
-    const uint64_t rows = ((n + most - 1) / most + 15) / 16 * 16;
-    return static_cast<uint32_t>(std::max<uint64_t>(rows, 128));
-}
-uint32_t part_count(uint64_t n, uint32_t most) { return static_cast<uint32_t>((n + part_rows(n, most) - 1) / part_rows(n, most)); }
-// parts of the weight gradients: 32 and 16 tiles times these are 256 blocks
-constexpr uint32_t kPartsW1 = 8, kPartsW2 = 16;
-uint32_t row_tiles(uint64_t n) { return static_cast<uint32_t>((n + kTile - 1) / kTile); }
-uint32_t col_blocks(uint64_t n) { return static_cast<uint32_t>((n + kColRows - 1) / kColRows); }
-
-}  // namespace
-
-uint64_t mlp_part_floats(uint64_t n)
-{
-    return static_cast<uint64_t>(part_count(n, kPartsW1)) * kMlpHidden * kMlpIn +
-           static_cast<uint64_t>(part_count(n, kPartsW2)) * kMlpHidden * kMlpHidden +
-           static_cast<uint64_t>(row_tiles(n)) * kMlpHidden + static_cast<uint64_t>(col_blocks(n)) * kColParts;
-}
-
 cudaError_t mlp_forward_f32(const MlpDevice& m, const MlpWork& w, const float* x, uint64_t n, cudaStream_t st)
 {
     const uint32_t H = kMlpHidden, R = static_cast<uint32_t>(n);
     if (!n) return cudaSuccess;
-    const dim3 grid(H / kTile, row_tiles(n));
+    const dim3 grid(H / kTile, mlp_parts(n).row_tiles);
     // h1 = relu(x . W1^T + b1), h2 = relu(h1 . W2^T + b2)
     gemm_f32_kernel<false, true, Epilogue::kBiasRelu>
         <<<grid, 256, 0, st>>>(x, kMlpIn, m.params + kOffW1, kMlpIn, w.h1, R, H, kMlpIn, kMlpIn, m.params + kOffB1,
@@ -911,23 +888,20 @@ cudaError_t mlp_loss_backward_f32(const MlpDevice& m, const MlpWork& w, const fl
     cudaError_t e = cudaMemsetAsync(w.loss, 0, 2 * sizeof(double), st);
     if (e != cudaSuccess) return e;
     loss_kernel<<<grid_for(n, 256), 256, 0, st>>>(w.s, y, weight, n, w.ds, w.loss);
-    const uint32_t z1 = part_count(n, kPartsW1), z2 = part_count(n, kPartsW2);
-    float* pw1 = w.parts;
-    float* pw2 = pw1 + static_cast<uint64_t>(z1) * H * kMlpIn;
-    float* pb1 = pw2 + static_cast<uint64_t>(z2) * H * H;
-    float* pcol = pb1 + static_cast<uint64_t>(row_tiles(n)) * H;
-    backward_columns_kernel<<<col_blocks(n), H, 0, st>>>(w.ds, w.h2, m.params, w.loss, n, w.dh2, pcol);
+    const MlpParts p = mlp_parts(n);
+    float *pw1 = w.parts, *pw2 = pw1 + p.w2, *pb1 = pw1 + p.b1, *pcol = pw1 + p.col;
+    backward_columns_kernel<<<p.col_blocks, H, 0, st>>>(w.ds, w.h2, m.params, w.loss, n, w.dh2, pcol);
     // dW2 = dh2^T h1
-    gemm_f32_kernel<true, false, Epilogue::kPartial><<<dim3(H / kTile, H / kTile, z2), 256, 0, st>>>(
-        w.dh2, H, w.h1, H, pw2, H, H, R, part_rows(n, kPartsW2), nullptr, nullptr, nullptr);
+    gemm_f32_kernel<true, false, Epilogue::kPartial><<<dim3(H / kTile, H / kTile, p.z2), 256, 0, st>>>(
+        w.dh2, H, w.h1, H, pw2, H, H, R, p.w2_rows, nullptr, nullptr, nullptr);
     // dh1 = dh2 W2 where h1 > 0; its column sums are db1
-    gemm_f32_kernel<false, false, Epilogue::kMask><<<dim3(H / kTile, row_tiles(n)), 256, 0, st>>>(
+    gemm_f32_kernel<false, false, Epilogue::kMask><<<dim3(H / kTile, p.row_tiles), 256, 0, st>>>(
         w.dh2, H, m.params + kOffW2, H, w.dh1, R, H, H, H, nullptr, w.h1, pb1);
     // dW1 = dh1^T x
-    gemm_f32_kernel<true, false, Epilogue::kPartial><<<dim3(kMlpIn / kTile, H / kTile, z1), 256, 0, st>>>(
-        w.dh1, H, x, kMlpIn, pw1, H, kMlpIn, R, part_rows(n, kPartsW1), nullptr, nullptr, nullptr);
-    reduce_gradient_kernel<<<(kMlpParams + 255) / 256, 256, 0, st>>>(pw1, z1, pw2, z2, pb1, row_tiles(n), pcol,
-                                                                    col_blocks(n), w.grad);
+    gemm_f32_kernel<true, false, Epilogue::kPartial><<<dim3(kMlpIn / kTile, H / kTile, p.z1), 256, 0, st>>>(
+        w.dh1, H, x, kMlpIn, pw1, H, kMlpIn, R, p.w1_rows, nullptr, nullptr, nullptr);
+    reduce_gradient_kernel<<<(kMlpParams + 255) / 256, 256, 0, st>>>(pw1, p.z1, pw2, p.z2, pb1, p.row_tiles, pcol,
+                                                                    p.col_blocks, w.grad);
     return cudaGetLastError();
 }
 

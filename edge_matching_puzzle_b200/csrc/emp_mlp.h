@@ -91,10 +91,47 @@ struct MlpWork {
     float* dh2 = nullptr;   // [rows][256]
     float* dh1 = nullptr;   // [rows][256]
     float* grad = nullptr;  // kMlpParams
-    float* parts = nullptr; // mlp_part_floats(rows) partial sums of the gradient
+    float* parts = nullptr; // mlp_part_floats(rows) partial sums of the gradient (MlpParts)
     double* loss = nullptr; // [2]: weighted loss sum, weight sum
 };
-uint64_t mlp_part_floats(uint64_t n);
+
+// Partial sums of a gradient over n rows, in MlpWork::parts: z1 of dW1 and z2 of dW2 (of w1_rows and
+// w2_rows rows each), then a row of db1 for each of row_tiles tiles, then col_blocks rows of
+// dw3 | db2 | db3.  The parts get no more numerous with the rows alone (2000 rows make 16 parts of
+// dW2, 2100 rows 15), so a workspace for up to `rows` rows is sized by mlp_part_floats, which
+// never falls: the most parts a gradient of that many rows or fewer has.
+constexpr uint32_t kMlpTile = 64, kMlpColRows = 32, kMlpColParts = 2 * kMlpHidden + 1;
+constexpr uint32_t kMlpPartRows = 128;                  // rows of a weight gradient's part, at least
+constexpr uint32_t kMlpPartsW1 = 8, kMlpPartsW2 = 16;   // at most: 32 and 16 tiles times these are 256 blocks
+struct MlpParts {
+    uint32_t z1, w1_rows, z2, w2_rows, row_tiles, col_blocks;
+    uint64_t w2, b1, col, end;  // offsets in floats (dW1's parts come first)
+};
+inline MlpParts mlp_parts(uint64_t n)
+{
+    auto split = [n](uint32_t most, uint32_t& count, uint32_t& rows) {
+        rows = static_cast<uint32_t>(((n + most - 1) / most + 15) / 16 * 16);
+        if (rows < kMlpPartRows) rows = kMlpPartRows;
+        count = static_cast<uint32_t>((n + rows - 1) / rows);
+    };
+    MlpParts p{};
+    split(kMlpPartsW1, p.z1, p.w1_rows);
+    split(kMlpPartsW2, p.z2, p.w2_rows);
+    p.row_tiles = static_cast<uint32_t>((n + kMlpTile - 1) / kMlpTile);
+    p.col_blocks = static_cast<uint32_t>((n + kMlpColRows - 1) / kMlpColRows);
+    p.w2 = static_cast<uint64_t>(p.z1) * kMlpHidden * kMlpIn;
+    p.b1 = p.w2 + static_cast<uint64_t>(p.z2) * kMlpHidden * kMlpHidden;
+    p.col = p.b1 + static_cast<uint64_t>(p.row_tiles) * kMlpHidden;
+    p.end = p.col + static_cast<uint64_t>(p.col_blocks) * kMlpColParts;
+    return p;
+}
+inline uint64_t mlp_part_floats(uint64_t rows)
+{
+    const MlpParts p = mlp_parts(rows);
+    const uint64_t few = (rows + kMlpPartRows - 1) / kMlpPartRows;  // parts of the fewest rows
+    const uint64_t z1 = few < kMlpPartsW1 ? few : kMlpPartsW1, z2 = few < kMlpPartsW2 ? few : kMlpPartsW2;
+    return p.end + (z1 - p.z1) * kMlpHidden * kMlpIn + (z2 - p.z2) * kMlpHidden * kMlpHidden;
+}
 // Forward of rows x[n][512] (f32) into h1, h2, s.
 cudaError_t mlp_forward_f32(const MlpDevice& m, const MlpWork& w, const float* x, uint64_t n, cudaStream_t stream);
 // Weighted logistic loss and its gradient with respect to every parameter (grad,
