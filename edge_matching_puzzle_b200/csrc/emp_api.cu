@@ -513,10 +513,10 @@ emp_status create_plan(const emp_puzzle* puzzles, uint32_t count, const emp_bt_c
                     ? emp::compact_smem_bytes(pl->max_levels, threads, pl->smem_tab_words, gs)
                     : emp::dfs_smem_bytes(pl->max_levels, pl->max_avail, threads, pl->smem_tab_words, pl->stack_mode);
             if (smem > static_cast<size_t>(smem_optin)) continue;
-            // (the compact kernel's limit and carve-out are the same for every plan, so that a plan
-            // created later never lowers them under an earlier one)
-            CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          pl->compact ? smem_optin : static_cast<int>(smem)));
+            // The limit and the carve-out belong to the kernel, not to the plan: they are the same for
+            // every plan (no search kernel has static shared memory), so that a plan created later
+            // never lowers them under an earlier one.
+            CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin));
             if (pl->compact && !gs && !pl->smem_tab_words)
                 CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 44));
             int per_sm = 0;
