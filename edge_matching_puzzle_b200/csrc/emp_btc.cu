@@ -538,12 +538,16 @@ __device__ __noinline__ bool split_state(const BtLaunch& P, uint32_t* out, const
 // levels are exhausted, ends its search above that level.  Measured on a B200 (split budget 64
 // without sharing, 256 with it): a 7x7 count of 2.3e6 placements 0.56 ms in 13 rounds -> 0.37 ms
 // in 5; 1/1024 of the tree above 3.84 -> 3.43 ms, 1/64 25.3 -> 25.7 ms at the same 30 -> 16 rounds.
+// A lane whose subtree a lower solution supersedes gives nothing away: the two would pass the work
+// to and fro, each for the 4096 steps between its looks at the flags.
 template <bool SM, int NW, int T>
 __device__ __noinline__ Search<NW> share_in_warp(const BtLaunch& P, Search<NW> s, uint32_t* stk)
 {
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t open = ~0u;
-    if (s.active)
+    const bool wanted =
+        !(P.stop_at_first && s.active && s.orig > *(volatile unsigned long long*)&P.first_item[puzzle<SM>(s)]);
+    if (s.active && wanted)
         for (uint32_t l = s.base; l < s.L; ++l)
             if (word_more(stk[l * T])) {
                 open = l;
@@ -617,6 +621,7 @@ __global__ void __launch_bounds__(T, (NW == 1 && SM ? (T == 128 ? 640 : 768) : 5
     idle<NW>(s);
     bool fix = false;          // the level's candidates still hold what its row's trials remove
     bool alive = true;
+    bool stopped = false;      // this lane saw the run's deadline or abort flag
     bool drained = false;      // warp-uniform: the input queue of this round is empty
     uint32_t iteration = 0;    // warp-uniform loop counter
     uint32_t alone = 0;        // warp-uniform: steps since the warp found the queue empty (no more
@@ -682,7 +687,8 @@ __global__ void __launch_bounds__(T, (NW == 1 && SM ? (T == 128 ? 640 : 768) : 5
         }
         if (drained && P.item_budget) {
             const unsigned busy = __ballot_sync(kFull, s.active);
-            if (busy && busy != kFull) {
+            // once the run stops, no lane takes on more
+            if (busy && busy != kFull && !__any_sync(kFull, stopped)) {
                 s = share_in_warp<SM, NW, T>(P, s, stk);
                 alive |= s.active;
             }
@@ -794,6 +800,7 @@ __global__ void __launch_bounds__(T, (NW == 1 && SM ? (T == 128 ? 640 : 768) : 5
             }
             const bool superseded =
                 P.stop_at_first && s.orig > *(volatile unsigned long long*)&P.first_item[puzzle<SM>(s)];
+            stopped |= stop;
             if (superseded || stop) {
                 account<SM, NW>(P, s);
                 if (stop) {

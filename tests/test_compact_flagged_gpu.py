@@ -47,3 +47,14 @@ def test_stop_at_first_counts_unsolvable_puzzles_whole(kw):
     got = native.bt_count_batch(handles, split_depth=4, stop_at_first=1, **kw)
     assert [(r.status, r.nodes, r.solutions) for r in got[1:]] == [(native.EMP_OK, w.nodes, 0) for w in want[1:]]
     assert list(got[0].first_solution)[:30] == list(want[0].first_board)[:30]
+
+
+@pytest.mark.parametrize("depth", [3, 12])
+def test_deadline_with_work_shared_in_warps(depth):
+    """Few subtrees, so that idle lanes take work all the time, and a split budget that hands none
+    back.  A lane looks at the clock every 4096 steps (2.3 ms on a full chip): the run ends within
+    20 ms of its deadline."""
+    pz = generate(8, 8, 4, 8, 0)  # 1.8e11 placements, over a second
+    r = native.bt_count(native.NativePuzzle(8, 8, pz.colors), split_depth=depth, timeout_ms=100, split_budget=1 << 20)
+    assert r.status == native.EMP_INCOMPLETE
+    assert 100 <= r.kernel_ms <= 120

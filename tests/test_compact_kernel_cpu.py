@@ -24,18 +24,22 @@ def kernel(tmp_path_factory):
                     os.path.join(ROOT, "tests", "compact_kernel_host.cpp"), os.path.join(CSRC, "emp_compact.cpp"),
                     os.path.join(CSRC, "emp_model.cpp")], check=True)
 
-    def run(puzzles, depth, smem=0, min_nw=1, budget=256, capacity=1 << 16, deadline=0, at_first=0, at_any=0):
+    def run(puzzles, depth, smem=0, min_nw=1, budget=256, capacity=1 << 16, deadline=0, at_first=0, at_any=0,
+            before=()):
         """Per puzzle (placements, solutions, incomplete) of its subtrees, then the run's clock,
-        rounds and rounds with a full queue; and the oracle's (placements, solutions)."""
+        rounds and rounds with a full queue; and the oracle's (placements, solutions).  before:
+        prefixes of the first puzzle that are queued ahead of its subtrees."""
+        records = [f"0 {len(p)} " + " ".join(str(t) for t in p) for p in before]
+        want = []
         text = [f"{int(smem)} {min_nw} {budget} {capacity} {deadline} {at_first} {at_any}", str(len(puzzles))]
-        records, want = [], []
         for i, p in enumerate(puzzles):
             text.append(f"{p.width} {p.height} " + " ".join(str(c) for q in p.colors for c in q))
             op = OraclePuzzle(p.width, p.height, p.colors)
             n, _, _, prefixes = op.expand(depth, max_prefixes=1 << 20)
             records += [f"{i} {depth} " + " ".join(str(t) for t in prefixes[j * depth:(j + 1) * depth])
                         for j in range(n)]
-            want.append(op.subtrees_parallel(prefixes, depth, 0, n, 4))
+            if not (deadline or at_any or before):  # else not searched out
+                want.append(op.subtrees_parallel(prefixes, depth, 0, n, 4))
         text.append(str(len(records)))
         out = subprocess.run([exe], input="\n".join(text + records) + "\n", capture_output=True, text=True,
                              check=True, timeout=120).stdout.splitlines()
@@ -87,3 +91,33 @@ def test_superseded_lanes_leave_other_puzzles_counts_whole(kernel, first, second
     assert want[1][1] == 0
     assert got[1] == want[1] + (0,)
     assert got[0][1]
+
+
+# ticks in which each of the four warps makes the steps between a lane's looks at the flags (4096, and a
+# fetch before and after): a step has at most four collectives
+LOOK = 4 * 4 * (4096 + 2 * 48)
+
+
+@pytest.mark.parametrize("kw", [{"budget": 1 << 20}, {"budget": 256, "capacity": 60}], ids=str)
+@pytest.mark.parametrize("board,depth", [((6, 6, 4, 2, 476079230), 5), ((6, 7, 2, 5, 916256161), 3)], ids=str)
+def test_deadline_ends_a_run_that_shares_work(kernel, board, depth, kw):
+    """Work that a lane at the deadline takes from a neighbour would go on for as long again."""
+    deadline = 40000
+    got, (clock, _, _), _ = kernel([generate(*board)], depth, deadline=deadline, **kw)
+    assert got[0][2] == 1  # incomplete
+    assert deadline < clock <= deadline + LOOK
+
+
+@pytest.mark.parametrize("stop", ["at_first", "at_any"])
+@pytest.mark.parametrize("board,depth", [((6, 6, 4, 2, 476079230), 5), ((6, 7, 2, 5, 916256161), 3)], ids=str)
+def test_first_solution_ends_a_run_that_shares_work(kernel, board, depth, stop):
+    """A first record that holds little but a solution, then subtrees that are not searched out."""
+    pz = generate(*board)
+    op = OraclePuzzle(pz.width, pz.height, pz.colors)
+    r, _ = op.run(node_limit=100000000)
+    assert r.solutions
+    kinds = {op.piece_of(k, i): i for k in range(3) for i in range(op.nb_kind(k))}
+    path = [(kinds[v >> 2] << 2) | (v & 3) for v in list(r.first_board)[: pz.nb_pieces]]
+    got, (clock, _, _), _ = kernel([pz], depth, budget=1 << 20, before=[path[:-4]], **{stop: 1})
+    assert got[0][1] >= 1
+    assert clock <= LOOK
