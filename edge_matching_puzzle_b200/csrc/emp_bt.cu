@@ -117,10 +117,16 @@ __global__ void expand_kernel(BtLaunch P, const uint16_t* __restrict__ parents,
                               unsigned long long* __restrict__ level_sols, int mode,
                               const uint8_t* __restrict__ frozen)
 {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n_parents;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t pz = parent_puzzle ? parent_puzzle[i] : 0u;
-        if (frozen && frozen[pz]) {
+    const uint32_t lane = threadIdx.x & 31u;
+    // (a warp's lanes make the same trips, so that the ballot names the lanes that count)
+    for (uint64_t warp_first = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x - lane; warp_first < n_parents;
+         warp_first += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t i = warp_first + lane;
+        const uint32_t pz = i < n_parents && parent_puzzle ? parent_puzzle[i] : 0u;
+        const bool carried = frozen && frozen[pz];
+        const unsigned counting = __ballot_sync(kFull, !mode && !carried && i < n_parents);
+        if (i >= n_parents) continue;
+        if (carried) {
             // this puzzle has enough subtrees: carry the prefix over, padded
             if (mode) {
                 const uint16_t* pre = parents + i * level;
@@ -141,9 +147,9 @@ __global__ void expand_kernel(BtLaunch P, const uint16_t* __restrict__ parents,
             counts[i] = cnt;
             // one addition for the lanes at work on the same puzzle (6.3 million parents of a 10x10
             // plan added to one address)
-            const unsigned peers = __match_any_sync(__activemask(), pz);
+            const unsigned peers = __match_any_sync(counting, pz);
             const uint32_t sum = __reduce_add_sync(peers, cnt);
-            if (sum && (threadIdx.x & 31u) == __ffs(peers) - 1) {
+            if (sum && lane == __ffs(peers) - 1) {
                 atomicAdd(&level_nodes[pz], (unsigned long long)sum);
                 if (last) atomicAdd(&level_sols[pz], (unsigned long long)sum);
             }
