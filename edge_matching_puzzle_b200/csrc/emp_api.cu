@@ -24,6 +24,15 @@ extern "C" uint32_t emp_abi_version(void) { return EMP_ABI_VERSION; }
 
 extern "C" const char* emp_last_error(void) { return emp::last_error().c_str(); }
 
+extern "C" emp_status emp_release_memory(int32_t device)
+{
+    emp::clear_error();
+    int ordinal = 0;
+    EMP_TRY(emp::select_device(device, &ordinal));
+    CUDA_TRY(emp::device_trim());
+    return EMP_OK;
+}
+
 extern "C" emp_status emp_generate_puzzle(uint32_t width, uint32_t height, uint32_t border_colors,
                                           uint32_t interior_colors, uint64_t seed, uint8_t* colours_out)
 {

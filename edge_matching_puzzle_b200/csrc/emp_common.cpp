@@ -113,6 +113,16 @@ void device_free(void* p, int device, uint64_t context)
     if (now != device) cudaSetDevice(now);
 }
 
+cudaError_t device_trim()
+{
+    const uint64_t id = context_id();
+    std::lock_guard<std::mutex> g(g_pool_lock);
+    auto it = pools().find(id);
+    if (it == pools().end() || !it->second.pool) return cudaSuccess;  // nothing was pooled here
+    const cudaError_t e = cudaStreamSynchronize(it->second.stream);
+    return e != cudaSuccess ? e : cudaMemPoolTrimTo(it->second.pool, 0);
+}
+
 std::string& last_error()
 {
     thread_local std::string message;

@@ -25,10 +25,12 @@ emp_status select_device(int device, int* ordinal);
 // mapping and unmapping them under the pool's limit took up to a second.  cudaMalloc and cudaFree cost 0.1 to 0.3 ms
 // a pair on a B200 and a one-shot count makes some thirty: a 5x5 count took 6.5 ms, 0.04 ms of
 // it on the device.  Like cudaFree, device_free waits for the device, so no stream still uses what
-// goes back.  Safe from several threads; a device reset in between is noticed.
+// goes back.  Safe from several threads; a device reset in between is noticed.  device_trim gives all
+// that is unused in the current device's pool back to the driver.
 constexpr uint64_t kPoolKeep = 2ull << 30, kPoolBlock = 512ull << 20;
 cudaError_t device_alloc(void** p, size_t bytes, int* device, uint64_t* context);
 void device_free(void* p, int device, uint64_t context);
+cudaError_t device_trim();
 
 // Owning device allocation (move-only).
 struct DeviceBuffer {

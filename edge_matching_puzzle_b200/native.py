@@ -146,6 +146,7 @@ SIGNATURES = {
     "emp_abi_version": (ctypes.c_uint32, []),
     "emp_glutton_wide_situation": (ctypes.c_int32, [ctypes.c_void_p, ctypes.POINTER(ctypes.c_uint32), ctypes.c_uint64]),
     "emp_last_error": (ctypes.c_char_p, []),
+    "emp_release_memory": (ctypes.c_int32, [ctypes.c_int32]),
     "emp_generate_puzzle": (ctypes.c_int32, [ctypes.c_uint32] * 4 + [ctypes.c_uint64, u8p]),
     "emp_puzzle_create": (ctypes.c_int32, [ctypes.POINTER(PuzzleDesc), ctypes.POINTER(ctypes.c_void_p)]),
     "emp_puzzle_destroy": (None, [ctypes.c_void_p]),
@@ -215,6 +216,11 @@ def check(status: int) -> int:
     if status < 0:
         raise EmpError(status, load().emp_last_error().decode())
     return status
+
+
+def release_memory(device: int = -1) -> None:
+    """emp_release_memory: device memory kept between calls goes back to the driver."""
+    check(load().emp_release_memory(device))
 
 
 def generate(width: int, height: int, border_colors: int, interior_colors: int, seed: int) -> List[List[int]]:

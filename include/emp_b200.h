@@ -50,6 +50,11 @@ uint32_t emp_abi_version(void);
 /* Message of the last failing call on this thread ("" when none). */
 const char *emp_last_error(void);
 
+/* Gives the device memory that the library keeps between calls (at most 2 GiB a device, for
+ * plans, searches and networks to come) back to the driver, for other processes to use.
+ * Live handles keep theirs.  device: ordinal, -1 = the current one. */
+emp_status emp_release_memory(int32_t device);
+
 /* Seeded puzzle generator of the project's workloads (splitmix64 stream):
  * frame-to-frame edges get colours 1..border_colors, other internal edges
  * border_colors+1..border_colors+interior_colors, outer edges 0; pieces are
