@@ -566,11 +566,13 @@ emp_status create_plan(const emp_puzzle* puzzles, uint32_t count, const emp_bt_c
         if (!resume) pl->rec_words = 4 + (pl->depth + 1) / 2;
         if (pl->stack_mode == emp::kStackGlobal32)
             CUDA_TRY(pl->stack.alloc(sizeof(uint32_t) * resident * emp::compact_stack_levels(pl->max_levels)));
-        // round queues: a thread hands its state back at most once a round, with an item per
-        // level that holds candidates: about 6 on an 8x8 board.  Room for 24; a thread that
-        // finds the queue full keeps its work.
+        // round queues: a thread hands its state back at most once a round, with an item per level
+        // that holds candidates, so an item a level never fills the queue.  Those are about 6 on an 8x8
+        // board, but above 24 on wide boards of few colours, where 24 a thread left the threads that
+        // found the queue full to search on alone: 12x8 of 3/5 colours split at level 6, 600 ms on a
+        // B200, 2.7e9 placements/s.
         pl->queue_words = emp::compact_state_words(pl->max_levels, pl->chdr.nw);
-        pl->capacity = resident * std::min<uint32_t>(24, pl->max_levels);
+        pl->capacity = resident * pl->max_levels;
         const uint64_t bytes = sizeof(uint32_t) * pl->queue_words * resident + sizeof(uint64_t) * pl->capacity;
         CUDA_TRY(pl->rec_a.alloc(bytes));
         CUDA_TRY(pl->rec_b.alloc(bytes));
@@ -942,7 +944,7 @@ emp_status count_one_plan(const emp_puzzle* puzzles, uint32_t count, const emp_b
 
 // Puzzles with a plan each, run up to four at a time on their plans' own streams: a search's last,
 // small rounds leave most of the chip idle, and another search's rounds fill it.  No more plans are
-// added once they hold 512 MiB (an 8x8 board's holds about 120 MB), so that the memory of later
+// added once they hold 768 MiB (an 8x8 board's holds about 180 MB), so that the memory of later
 // groups comes from the pool.  A plan that cannot be made beside others is made again alone.
 // Measured on a B200, 1/64 of four 8x8 trees (2.95e9 placements), a whole call:
 // 37.6 ms one after the other, 31.6 ms side by side.
@@ -950,7 +952,7 @@ emp_status count_side_by_side(const emp_puzzle* puzzles, uint32_t count, const e
                               emp_bt_result* results)
 {
     constexpr uint32_t kSide = 4;
-    constexpr uint64_t kSideBytes = 512ull << 20;
+    constexpr uint64_t kSideBytes = 768ull << 20;
     bool alone = false;
     for (uint32_t done = 0; done < count;) {
         std::vector<std::unique_ptr<emp_bt_plan_t>> plans;
