@@ -1291,6 +1291,7 @@ __global__ void reset_kernel(BtLaunch P, uint32_t n_puzzles)
         P.first_records[i].lock = P.first_lock_init;
         P.first_records[i].missed = 0;
         P.first_records[i].has = 0;
+        P.first_records[i].version = 0;
     }
 }
 

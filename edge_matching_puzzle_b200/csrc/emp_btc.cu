@@ -426,14 +426,40 @@ __device__ __forceinline__ void load_record(const BtLaunch& P, Search<NW>& s, co
     start_search<NW>(s, len);
 }
 
+// whether this solution's path comes before the recorded one
+template <bool SM, int NW, int T>
+__device__ __forceinline__ bool path_before(const BtLaunch& P, const Search<NW>& s, const uint32_t* stk,
+                                            const FirstRecord* r)
+{
+    for (uint32_t l = 0; l < levels<SM>(P, s); ++l) {
+        const uint32_t mine = word_transition<SM, NW>(P, s, stk[l * T]);
+        const uint32_t theirs = *reinterpret_cast<const volatile uint16_t*>(&r->t[l]);
+        if (mine != theirs) return mine < theirs;
+    }
+    return false;
+}
+
 // Keeps the lexicographically smallest solution path of each puzzle, as record_solution of
-// emp_bt.cu does (bounded wait for the record's lock).
+// emp_bt.cu does (bounded wait for the record's lock).  The record only ever improves, so a path
+// that does not come before an unchanged copy of it needs no lock: `version` is odd while the
+// record is written.  Lanes that share the lowest subtree find its solutions at once, and on boards
+// with millions of them all waited for the lock: 7x7 of 1/2 colours, split at level 6, counted 4e8
+// placements/s and ended 0.56 s after a deadline of 0.2 s; now 4.4e10 and 7 ms.
 template <bool SM, int NW, int T>
 __device__ __forceinline__ void record_solution(const BtLaunch& P, const Search<NW>& s, const uint32_t* stk)
 {
     FirstRecord* r = P.first_records + puzzle<SM>(s);
-    atomicMin(&P.first_item[puzzle<SM>(s)], (unsigned long long)s.orig);
-    if (s.orig > *(volatile unsigned long long*)&P.first_item[puzzle<SM>(s)]) return;
+    // (the lowest subtree only falls: mostly a look is enough)
+    const unsigned long long lowest = *(volatile unsigned long long*)&P.first_item[puzzle<SM>(s)];
+    if (s.orig > lowest) return;
+    if (s.orig < lowest && atomicMin(&P.first_item[puzzle<SM>(s)], (unsigned long long)s.orig) < s.orig) return;
+    const uint32_t version = *(volatile unsigned int*)&r->version;
+    if (version && !(version & 1u)) {
+        __threadfence();
+        const bool before = path_before<SM, NW, T>(P, s, stk, r);
+        __threadfence();
+        if (!before && *(volatile unsigned int*)&r->version == version) return;
+    }
     const uint64_t give_up = global_ns() + P.first_lock_wait_ns;
     while (atomicCAS(&r->lock, 0u, 1u) != 0u) {
         if (global_ns() > give_up) {
@@ -444,31 +470,30 @@ __device__ __forceinline__ void record_solution(const BtLaunch& P, const Search<
         __nanosleep(64);
     }
     __threadfence();
-    bool better = !r->has;
-    if (!better) {
-        for (uint32_t l = 0; l < levels<SM>(P, s); ++l) {
-            const uint32_t mine = word_transition<SM, NW>(P, s, stk[l * T]), theirs = r->t[l];
-            if (mine != theirs) {
-                better = mine < theirs;
-                break;
-            }
-        }
-    }
-    if (better) {
+    if (!r->has || path_before<SM, NW, T>(P, s, stk, r)) {
+        atomicAdd(&r->version, 1u);
+        __threadfence();
         for (uint32_t l = 0; l < levels<SM>(P, s); ++l)
             r->t[l] = static_cast<uint16_t>(word_transition<SM, NW>(P, s, stk[l * T]));
         r->has = 1;
+        __threadfence();
+        atomicAdd(&r->version, 1u);
     }
     __threadfence();
     atomicExch(&r->lock, 0u);
 }
 
-// A solution's whole path is on the stack (its last piece's word included).
+// A solution's whole path is on the stack (its last piece's word included).  who: the lanes of the
+// warp that found one at this step.  They are counted together, for an addition each to one address
+// and one to the lowest subtree took 40 % of a search in which 1.2 % of the placements are solutions
+// (8x8 of 1/3 colours: 3.0e10 placements/s so, 5.0e10 now).
 template <bool SM, int NW, int T>
 __device__ __noinline__ void solution_found(const BtLaunch& P, const Search<NW> s, const uint32_t* stk,
-                                            uint32_t placed)
+                                            uint32_t placed, unsigned who)
 {
-    atomicAdd(&P.totals[2 * puzzle<SM>(s) + 1], 1ull);
+    const unsigned peers = SM ? who : __match_any_sync(who, s.pz);
+    if ((threadIdx.x & 31u) == __ffs(peers) - 1)
+        atomicAdd(&P.totals[2 * puzzle<SM>(s) + 1], static_cast<unsigned long long>(__popc(peers)));
     if (P.item_nodes) atomicAdd(&P.item_sols[s.orig], 1ull);
     record_solution<SM, NW, T>(P, s, stk);
     if (P.sols) {
@@ -765,9 +790,9 @@ __global__ void __launch_bounds__(T, (NW == 1 && SM ? (T == 128 ? 640 : 768) : 5
                     s.entries = r.entries;
                 }
             }
-            if (__any_sync(kFull, solved)) {
+            if (const unsigned who = __ballot_sync(kFull, solved)) {
                 if (solved) {
-                    solution_found<SM, NW, T>(P, s, stk, placed);
+                    solution_found<SM, NW, T>(P, s, stk, placed, who);
                 }
                 __syncwarp();
             }

@@ -30,6 +30,9 @@ constexpr uint32_t kThreads = 128;
 struct Warp {
     uint64_t value[2][32];
     uint32_t arrived = 0, phase = 0;
+    uint64_t some[32];  // a collective of some of the lanes
+    unsigned peers[32];
+    uint32_t some_arrived = 0, some_phase = 0;
 };
 struct Lane {
     ucontext_t first;
@@ -131,6 +134,25 @@ inline unsigned __ballot_sync(unsigned, bool v)
 inline int __any_sync(unsigned m, bool v) { return __ballot_sync(m, v) != 0; }
 template <class T>
 T __shfl_sync(unsigned, T v, int from) { return static_cast<T>(exchange(v)[from & 31]); }
+template <class T>
+unsigned __match_any_sync(unsigned mask, T v)
+{
+    // the lanes of the mask alone meet here
+    Warp& w = g_warps[g_tid / 32];
+    const uint32_t phase = w.some_phase;
+    w.some[g_tid % 32] = v;
+    if (++w.some_arrived == static_cast<uint32_t>(__builtin_popcount(mask))) {
+        for (int l = 0; l < 32; ++l) {
+            w.peers[l] = 0;
+            for (int k = 0; k < 32; ++k) w.peers[l] |= static_cast<unsigned>((mask >> k & 1u) && w.some[k] == w.some[l]) << k;
+        }
+        w.some_arrived = 0;
+        ++w.some_phase;
+    } else {
+        while (*const_cast<volatile uint32_t*>(&w.some_phase) == phase) yield();
+    }
+    return w.peers[g_tid % 32];
+}
 inline int __popc(unsigned v) { return __builtin_popcount(v); }
 inline int __ffs(unsigned v) { return __builtin_ffs(static_cast<int>(v)); }
 inline int __ffsll(long long v) { return __builtin_ffsll(v); }
