@@ -604,17 +604,39 @@ __device__ __forceinline__ bool dfs_step(const BtLaunch& P, ThreadItem& s, S& st
     return true;
 }
 
+// whether this solution's path comes before the recorded one
+template <class S>
+__device__ __forceinline__ bool path_before(const ThreadItem& s, const S& stk, const FirstRecord* r)
+{
+    for (uint32_t l = 0; l < s.n; ++l) {
+        const uint32_t mine = stk.t(l), theirs = *reinterpret_cast<const volatile uint16_t*>(&r->t[l]);
+        if (mine != theirs) return mine < theirs;
+    }
+    return false;
+}
+
 // Keeps the lexicographically smallest solution path of each puzzle: in the
 // reference's visiting order (ascending candidate bit at every level) that is
-// its first solution.  The lock is held for a few hundred cycles; the wait for
-// it is bounded in time (first_lock_wait_ns of %globaltimer) and a thread that
-// gives up flags the record as missed, which the host reports as EMP_FIRST_LOST.
+// its first solution.  The record only ever improves, so a path that does not come before an
+// unchanged copy of it (`version` is odd while it is written) needs no lock; else all threads on
+// the lowest subtree of a board with millions of solutions wait for one another (10x10 of 1/2
+// colours, split at level 6: 9.5e8 placements/s and 160 ms past a deadline, 1.6e10 and 5 ms so).
+// The lock is held for a few hundred cycles; the wait for it is bounded in time (first_lock_wait_ns
+// of %globaltimer) and a thread that gives up flags the record as missed, which the host reports
+// as EMP_FIRST_LOST.
 template <class S>
 __device__ void record_solution(const BtLaunch& P, const ThreadItem& s, const S& stk)
 {
     FirstRecord* r = P.first_records + s.pz;
     atomicMin(&P.first_item[s.pz], (unsigned long long)s.orig);
     if (s.orig > *(volatile unsigned long long*)&P.first_item[s.pz]) return;
+    const uint32_t version = *(volatile unsigned int*)&r->version;
+    if (version && !(version & 1u)) {
+        __threadfence();
+        const bool before = path_before(s, stk, r);
+        __threadfence();
+        if (!before && *(volatile unsigned int*)&r->version == version) return;
+    }
     const uint64_t give_up = global_ns() + P.first_lock_wait_ns;
     while (atomicCAS(&r->lock, 0u, 1u) != 0u) {
         if (global_ns() > give_up) {
@@ -625,19 +647,13 @@ __device__ void record_solution(const BtLaunch& P, const ThreadItem& s, const S&
         __nanosleep(64);
     }
     __threadfence();
-    bool better = !r->has;
-    if (!better) {
-        for (uint32_t l = 0; l < s.n; ++l) {
-            const uint32_t mine = stk.t(l), theirs = r->t[l];
-            if (mine != theirs) {
-                better = mine < theirs;
-                break;
-            }
-        }
-    }
-    if (better) {
+    if (!r->has || path_before(s, stk, r)) {
+        atomicAdd(&r->version, 1u);
+        __threadfence();
         for (uint32_t l = 0; l < s.n; ++l) r->t[l] = static_cast<uint16_t>(stk.t(l));
         r->has = 1;
+        __threadfence();
+        atomicAdd(&r->version, 1u);
     }
     __threadfence();
     atomicExch(&r->lock, 0u);

@@ -24,7 +24,7 @@ struct FirstRecord {
     unsigned int lock;
     unsigned int missed;    // a writer gave up waiting for the lock
     unsigned int has;
-    unsigned int version;   // compact search: changes of the record so far, twice; odd during one
+    unsigned int version;   // changes of the record so far, twice; odd during one
     uint16_t t[256];        // transition per level
 };
 

@@ -62,9 +62,19 @@ def test_puzzles_of_one_plan():
         _check(r, w, b[0] * b[1])
 
 
+@pytest.mark.parametrize("placement", [1, 3, 4])
+@pytest.mark.parametrize("board", BOARDS[:3], ids=str)
+def test_bitfield_search(board, placement):
+    npz, want = _puzzle(board)
+    for budget in (1, 0):
+        _check(native.bt_count(npz, split_depth=4, stack_placement=placement, split_budget=budget), want,
+               board[0] * board[1])
+
+
+@pytest.mark.parametrize("placement", [0, 3])
 @pytest.mark.parametrize("board", [(7, 7, 1, 2, 0), (10, 10, 1, 2, 1)], ids=str)
-def test_deadline(board):
+def test_deadline(board, placement):
     npz = native.NativePuzzle(board[0], board[1], generate(*board).colors)
-    r = native.bt_count(npz, split_depth=6, timeout_ms=200)
+    r = native.bt_count(npz, split_depth=6, timeout_ms=200, stack_placement=placement)
     assert r.status == native.EMP_INCOMPLETE
     assert 200 <= r.kernel_ms <= 300  # 4096 steps past the deadline at most; all lanes in a row took 560 to 700 ms
