@@ -388,6 +388,19 @@ emp_status resume_records(const emp_puzzle_t& pz, const uint16_t* situation, uin
     return EMP_OK;
 }
 
+// Whether replaying the trials of flagged rows over sets of several words costs the compact search
+// more than the bitfield search's wider sets cost that: measured on a B200, placements/s of the
+// bitfield against the compact search, 200 ms split at level 6, two words: sets of up to four
+// 64-bit words (9x9 to 12x8 and 10x10 boards of 2 or 3 border and 3 to 5 interior colours) 2.6e10 ..
+// 3.1e10 against 1.9e10 .. 2.3e10, five and six words 1.7e10 .. 1.9e10 against 1.9e10 .. 2.7e10; four
+// words: six and seven words (11x11, 12x12) 1.4e10 .. 1.7e10 against 0.9e10 .. 1.4e10, eight words
+// 1.0e10 .. 1.4e10 against 1.3e10 .. 1.4e10, more 0.6e10 .. 0.9e10 against 1.3e10 .. 1.4e10.  Without
+// flagged rows, and with one word, the compact search is the faster one throughout.
+bool replay_costs_more(const emp::CompactHeader& h, uint32_t max_kw)
+{
+    return h.flagged && h.nw > 1 && max_kw <= (h.nw == 2 ? 4u : 7u);
+}
+
 // Decides for the compact search and uploads its tables: every puzzle of the plan has them,
 // and in a plan of several puzzles every centre space is one word.  Measured on a B200, batches
 // of sides 4..9 in 2 s: with one 9x9 puzzle of two words the whole plan runs the two-word kernel
@@ -398,6 +411,10 @@ emp_status upload_compact(emp_bt_plan_t& pl)
     pl.compact = pl.cfg.stack_placement == 0;
     for (emp_puzzle p : pl.puzzles)
         if (p->compact.empty() || (pl.puzzles.size() > 1 && p->compact[0] != 1)) pl.compact = false;
+    if (!pl.compact) return EMP_OK;
+    emp::CompactHeader first;
+    std::memcpy(&first, pl.puzzles[0]->compact.data(), sizeof(first));
+    pl.compact = !replay_costs_more(first, pl.max_kw);
     if (!pl.compact) return EMP_OK;
     std::vector<uint32_t> blob;
     std::vector<uint64_t> offs;

@@ -184,6 +184,7 @@ std::vector<uint32_t> build_compact(const PuzzleModel& m, const std::vector<Leve
     std::vector<uint16_t> entries;
     std::vector<uint32_t> idrow(rows, 0);  // 1 + index into clears of flagged rows
     std::vector<uint64_t> clears;
+    uint32_t flagged = 0;
     std::vector<uint8_t> piece(static_cast<size_t>(2) * cap, 0);
     auto piece_bits = [&](uint32_t s, size_t i) { return ((uint64_t(1) << need[s][i]) - 1) << (first[s][i] & 63u); };
     for (uint32_t s = 0; s < 2; ++s)
@@ -226,6 +227,7 @@ std::vector<uint32_t> build_compact(const PuzzleModel& m, const std::vector<Leve
                 }
             }
             if (flag) {
+                ++flagged;
                 mask[static_cast<size_t>(r) * nw + nw - 1] |= uint64_t(1) << 63;
                 const size_t at = clears.size();
                 clears.resize(at + static_cast<size_t>(cap) * nw, 0);
@@ -254,6 +256,7 @@ std::vector<uint32_t> build_compact(const PuzzleModel& m, const std::vector<Leve
     h.width = width;
     h.nborder = nborder;
     h.rows = rows;
+    h.flagged = flagged;
     h.desc = place(4 * (n + 1), 4);
     h.slots = place(8 * cap, 4);
     h.rows_off = place(static_cast<size_t>(rows) * rb / 4, 4);

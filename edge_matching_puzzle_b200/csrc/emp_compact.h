@@ -63,7 +63,8 @@ struct CompactHeader {
     uint32_t nborder;    // border pieces: kind index of the first corner in space 1
     uint32_t words;      // blob size (multiple of 4)
     uint32_t rows;
-    uint32_t pad[2];
+    uint32_t flagged;    // rows whose trials are replayed
+    uint32_t pad;
 };
 
 constexpr uint32_t row_bytes(uint32_t nw) { return nw == 1 ? 16 : (nw == 2 ? 32 : 48); }
