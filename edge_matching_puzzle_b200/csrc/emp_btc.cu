@@ -790,7 +790,8 @@ __global__ void __launch_bounds__(T, (NW == 1 && SM ? (T == 128 ? 640 : 768) : 5
                     s.entries = r.entries;
                 }
             }
-            if (const unsigned who = __ballot_sync(kFull, solved)) {
+            if (__any_sync(kFull, solved)) {
+                const unsigned who = __ballot_sync(kFull, solved);
                 if (solved) {
                     solution_found<SM, NW, T>(P, s, stk, placed, who);
                 }
