@@ -192,10 +192,10 @@ __device__ uint64_t block_exclusive_scan(uint64_t v, uint64_t* sh, uint64_t& tot
 // [2] the buffer they are in.
 constexpr uint32_t kFewThreads = 1024;
 
-__global__ void __launch_bounds__(kFewThreads) expand_few_kernel(BtLaunch P, uint16_t* buf0, uint16_t* buf1, uint32_t* pz0, uint32_t* pz1,
-                                                                 uint32_t n_roots, uint32_t max_level, uint32_t capacity,
-                                                                 unsigned long long* level_nodes,
-                                                                 unsigned long long* level_sols, uint32_t* out)
+__global__ void __launch_bounds__(kFewThreads)
+    expand_few_kernel(BtLaunch P, uint16_t* buf0, uint16_t* buf1, uint32_t* pz0, uint32_t* pz1, uint32_t n_roots,
+                      uint32_t max_level, uint32_t capacity, unsigned long long* level_nodes,
+                      unsigned long long* level_sols, uint32_t* out)
 {
     __shared__ uint64_t sh[32];
     uint32_t np = n_roots, which = 0, level = 0;

@@ -12,9 +12,10 @@
 // A step of a warp runs (1) a pop for the lanes whose level is exhausted, (2) the next candidate
 // for all lanes that have one, (3) the way down for those whose candidate allows it.  A lane
 // whose pop found nothing left there pops again at the next step.  What is rare (flagged rows,
-// solutions) is left to a vote of the warp, so the common path has two divergent regions.  The set left at a level is not stored: a pop recomputes it as
-// the row AND the availability (which is the level's entry availability again) above the
-// slot placed there, with the trials of flagged rows replayed (emp_compact.h).
+// solutions) is left to a vote of the warp, so the common path has two divergent regions.  The set
+// left at a level is not stored: a pop recomputes it as the row AND the availability (which is the
+// level's entry availability again) above the slot placed there, with the trials of flagged rows
+// replayed (emp_compact.h).
 //
 // The stack keeps one 32-bit word a level:
 //   south colour | slot << 8 | more << 16 | space << 17 | (byte offset of the row / 16) << 18
@@ -24,7 +25,8 @@
 // What bounds it: integer instructions (ALU pipe 78.5 % and issue slots 76.8 % busy in the main
 // rounds on a B200, 21 lanes in an instruction, 20 warps an SM, which hide the shared-memory
 // latency); 30 of 32 lanes have work at a step, 22 of them a candidate.  Measured, 1/64 of the
-// 8x8 tree of 4 border / 8 interior colours, seed 0 (2.77e9 placements): 62.9 ms with dfs_kernel (4.4e10 placements/s), 23.4 ms here (1.18e11/s).
+// 8x8 tree of 4 border / 8 interior colours, seed 0 (2.77e9 placements): 62.9 ms with dfs_kernel
+// (4.4e10 placements/s), 23.3 ms here (1.19e11/s).
 // 128-thread blocks, five an SM, let a thread have its 90 registers: 20 warps at 23.4 ms, where 24 warps
 // of 80 registers (256-thread blocks) take 24.2 ms and 16 of 128 registers 24.0 ms; on
 // 1/1024 of the tree 3.07 against 3.4 ms.  Tried and slower: selects in place of the step's two
@@ -524,7 +526,11 @@ __device__ __forceinline__ void account(const BtLaunch& P, const Search<NW>& s)
 
 // Hands the remaining work of the thread to the next round: its state, in the slot that is this
 // thread's own, and one item per level that still holds candidates (the more bits say which).
-// Returns false when the item queue is full (the thread then keeps the work).
+// Returns false when the item queue is full (the thread then keeps the work; the plans' queues hold
+// every open level, so theirs never fill).  A state slot is written once a round, since items point
+// to it: a lane that handed back may take work again from a neighbour that could not
+// (share_in_warp), but its own next attempt fails too, for the queue's tail never falls, and once a
+// neighbour did not fit nothing fits.  A rule that hands back at another time has to keep that.
 template <bool SM, int NW, int T>
 __device__ __noinline__ bool split_state(const BtLaunch& P, uint32_t* out, const Search<NW> s, const uint32_t* stk)
 {
@@ -631,7 +637,8 @@ __device__ __noinline__ Search<NW> share_in_warp(const BtLaunch& P, Search<NW> s
 // cancellation and stop-at-first flags are those of dfs_kernel.  Work goes back to the queue for
 // the next round once a warp has searched on for the split budget after the queue ran empty.
 template <int NW, bool SM, bool GS, int T, int kStepsPerFetch>
-__global__ void __launch_bounds__(T, (NW == 1 && SM ? (T == 128 ? 640 : 768) : 512) / T) dfs_compact_kernel(const __grid_constant__ BtLaunch P)
+__global__ void __launch_bounds__(T, (NW == 1 && SM ? (T == 128 ? 640 : 768) : 512) / T)
+    dfs_compact_kernel(const __grid_constant__ BtLaunch P)
 {
     using TB = Tab<SM, NW>;
     const uint32_t tid = threadIdx.x, lane = tid & 31;

@@ -22,9 +22,9 @@ emp_status select_device(int device, int* ordinal);
 // Device memory comes from a pool of this library's own, one per device, that holds on to at most
 // kPoolKeep bytes of freed memory between calls (the driver takes unused pool memory back when an
 // allocation elsewhere in the process would fail).  Blocks above kPoolBlock are not pooled:
-// mapping and unmapping them under the pool's limit took up to a second.  cudaMalloc and cudaFree cost 0.1 to 0.3 ms
-// a pair on a B200 and a one-shot count makes some thirty: a 5x5 count took 6.5 ms, 0.04 ms of
-// it on the device.  Like cudaFree, device_free waits for the device, so no stream still uses what
+// mapping and unmapping them under the pool's limit took up to a second.  cudaMalloc and cudaFree cost
+// 0.1 to 0.3 ms a pair on a B200 and a one-shot count makes some thirty: a 5x5 count took 6.5 ms,
+// 0.04 ms of it on the device.  Like cudaFree, device_free waits for the device, so no stream still uses what
 // goes back.  Safe from several threads; a device reset in between is noticed.  device_trim gives all
 // that is unused in the current device's pool back to the driver.
 constexpr uint64_t kPoolKeep = 2ull << 30, kPoolBlock = 512ull << 20;

@@ -30,8 +30,9 @@
 // each position), and compared as 16-bit pairs.  The candidates of a pass are dealt out evenly by
 // rank; each thread finds its own.
 //
-// What bounds it: the trials' instructions (about 85 a word of eight pieces) and the statistics
-// and barrier of each pass, which every block repeats.  Measured on a B200, whole calls: 16x16
+// What bounds it: instructions, of the trials (about 85 a word of eight pieces) and of the statistics
+// that every block repeats in each pass (16x16, 20 pushes: ALU pipe 65 %, issue slots 58 % busy, 30.7
+// lanes in an instruction), and the block barriers between the steps of a pass (the top stall).  Measured on a B200, whole calls: 16x16
 // (5/17 colours, 300 pushes, 148 blocks) 165 ms with a warp a trial, shuffles for every sum,
 // full scans for the lists and a work counter; 42 ms with a group of lanes a trial, 320
 // instructions in each lane; 28 ms now, 22 us a pass of 45 000 trials.  8x8 on one block (150
@@ -177,9 +178,10 @@ __device__ __forceinline__ uint32_t candidate_of_rank(const GmSmem& sm, uint32_t
     return (j << 10) | (w << 5) | b;
 }
 
-// Per-pass statistics of the current level (block-wide).  Returns whether an info is empty.  The six smallest and largest A[j]-N[j][q] of a piece are found by visiting the
-// infos in order of A: N is at most 4, so the visit ends once no later info can enter the list (a
-// scan of all 256 infos for each piece and list took most of the statistics' time).
+// Per-pass statistics of the current level (block-wide).  Returns whether an info is empty.  The six
+// smallest and largest A[j]-N[j][q] of a piece are found by visiting the infos in order of A: N is at
+// most 4, so the visit ends once no later info can enter the list (a scan of all 256 infos for each
+// piece and list took most of the statistics' time).
 __device__ bool level_statistics(GmSmem& sm, uint32_t n, uint32_t nb, uint32_t width, uint32_t tid)
 {
     const uint32_t lane = tid & 31, warp = tid >> 5, j = tid >> 2, w0 = 8 * (tid & 3u);
